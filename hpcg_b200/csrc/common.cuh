@@ -238,6 +238,12 @@ struct Level {
   int wf_tpu = 0;
   unsigned* wf_done = nullptr;
   int wf = 0;
+  // the columns are exactly the 27-point stencil's (every neighbour inside the
+  // grid present), and the injected rows are the even points: what the
+  // one-launch small levels (tail.cuh) rely on instead of reading them
+  bool geo = false;
+  bool geo_f2c = false;
+  double* valt = nullptr;  // FP64 values in the layout tail.cuh reads (small levels only, built on first use)
 };
 
 struct Context;
@@ -266,6 +272,7 @@ struct hpcg_b200_problem {
   // and whether b still holds it (every other load into b clears the flag)
   double* b_kept_host;
   bool b_kept;
+  int tail_first[2];  // first level run by the one-launch small end of the V-cycle (tail.cuh), [FP64, FP32]; -1: not decided
   int host_reuse;  // hpcg_b200_cg may skip sending an unchanged b and a zero x (hpcg_b200_set_host_reuse)
 };
 
@@ -466,6 +473,19 @@ inline int sink_of(const Level& L) { return L.n + L.next; }
 // true for a rank of a run over several ranks: the single-rank entry points
 // refuse it (its halo would never be exchanged)
 inline bool is_rank(const hpcg_b200_problem* p) { return p->geom != nullptr && p->geom->size > 1; }
+
+// The small end of the V-cycle in one launch (tail.cu). tail_first: the first
+// level it runs (p->nlev: none). The launchers return false where nothing was
+// queued (the launch was refused, and is not tried again): the caller runs the
+// phases. tail_step: one symmetric Gauss-Seidel step on level l, x entering
+// nonzero; taken where tail_step_ok.
+// tail_values: (re)builds a small level's copy of its FP64 values.
+int tail_first(hpcg_b200_problem* p, bool f32);
+int tail_values(hpcg_b200_problem* p, int l);
+bool tail_step_ok(hpcg_b200_problem* p, int l);
+bool tail_vcycle(hpcg_b200_problem* p, int l, const double* r, double* x);
+bool tail_vcycle(hpcg_b200_problem* p, int l, const float* r, float* x);
+bool tail_step(hpcg_b200_problem* p, int l, const double* r, double* x);
 
 // natural <-> colour order vector movement (solver.cu)
 int load_vector(hpcg_b200_problem* p, int level, const double* src_natural, double* dst_colour);

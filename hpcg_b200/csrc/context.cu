@@ -264,6 +264,7 @@ int stream_sync(Context* c) {
     *f = 0;
     set_error_text(code == 5   ? "a device-side wait gave up (bounded wait at the batched iteration's grid barrier)"
                    : code == 6 ? "a device-side wait gave up (bounded wait of a wavefront sweep on its dependencies)"
+                  : code == 7 ? "a device-side wait gave up (bounded wait between two phases of the one-launch small levels)"
                                : "a device-side wait gave up (bounded mbarrier wait of the bulk-copy pipeline)");
     return HPCG_B200_ERR_TIMEOUT;
   }

@@ -43,6 +43,7 @@ hpcg_b200_problem* new_problem(int device, Context* c) {
   const char* reuse = std::getenv("HPCG_B200_HOST_REUSE");
   p->host_reuse = reuse && reuse[0] == '0' ? 0 : 1;
   for (int l = 0; l < kMaxLevels; ++l) p->lev[l] = Level();
+  p->tail_first[0] = p->tail_first[1] = -1;
   return p;
 }
 
@@ -370,7 +371,7 @@ int free_problem(hpcg_b200_problem* p) {
   for (int l = 0; l < kMaxLevels; ++l) {
     Level& L = p->lev[l];
     void* ptrs[] = {L.val, L.col, L.val32, L.col32, L.new2old, L.old2new, L.f2c, L.tf, L.tq, L.r, L.x, L.r32, L.x32,
-                    L.wave_rows, L.colp, L.wf_done};
+                    L.wave_rows, L.colp, L.wf_done, L.valt};
     for (void* q : ptrs) dev_free(q);
     delete[] L.wave_start;
     delete L.maps;
@@ -447,6 +448,7 @@ int generate_impl(int nx, int ny, int nz, int nlevels, int device, const RankGeo
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) { set_error("generate", e); status = status_of(e); }
+    L.geo = L.geo_f2c = G.size == 1;
   }
   for (int l = 0; l + 1 < nlevels && status == HPCG_B200_OK; ++l) status = build_transfer(p, l);
   for (int l = 0; l < nlevels && status == HPCG_B200_OK; ++l) status = upload_plan(p, l, sends[l]);
@@ -501,6 +503,7 @@ int hpcg_b200_optimize(const hpcg_b200_level_desc* desc, int nlevels, int device
     std::vector<int> col((size_t)kSlots * pitch, n);
     std::vector<int> n2o(n), o2n(n);
     std::atomic<int> bad(0);
+    std::atomic<bool> full(true);  // every neighbour inside the grid is present
     parallel_for(n, [&](int64_t b, int64_t e) {
       for (int64_t i = b; i < e; ++i) {
         const int ix = (int)(i % d.nx), iy = (int)((i / d.nx) % d.ny), iz = (int)(i / ((int64_t)d.nx * d.ny));
@@ -522,9 +525,13 @@ int hpcg_b200_optimize(const hpcg_b200_level_desc* desc, int nlevels, int device
           col[(size_t)k * pitch + q] = g.old2new(ix + dx, iy + dy, iz + dz);
         }
         if (!(seen & (1u << kDiagSlot))) bad = 1;
+        auto reach = [](int i, int n) { return 1 + (i > 0) + (i + 1 < n); };
+        if (cnt != reach(ix, d.nx) * reach(iy, d.ny) * reach(iz, d.nz)) full = false;
       }
     });
     if (bad) { status = HPCG_B200_ERR_UNSUPPORTED; break; }
+    L.geo = full;
+    L.geo_f2c = true;
     status = alloc_n(p, &L.val, kSlots * pitch);
     if (!status) status = alloc_n(p, &L.col, kSlots * pitch);
     if (!status) status = alloc_n(p, &L.new2old, n);
@@ -546,6 +553,7 @@ int hpcg_b200_optimize(const hpcg_b200_level_desc* desc, int nlevels, int device
         const int ff = d.f2c[natc];
         if (ff < 0 || ff >= n) { bad = 1; break; }
         f[qc] = o2n[ff];
+        if (f[qc] != g.old2new(2 * cx, 2 * cy, 2 * cz)) L.geo_f2c = false;
       }
       if (bad) { status = HPCG_B200_ERR_ARG; break; }
       status = alloc_n(p, &L.f2c, nc);
@@ -661,6 +669,7 @@ int hpcg_b200_set_diagonal(hpcg_b200_problem* p, const double* diagonal) {
   }
   k_set_diag<<<grid_for(c, L.n, 256, 8), 256, 0, c->stream>>>(src, L.old2new, L.val + kDiagSlot * L.pitch, L.n);
   HB_CK(cudaGetLastError());
+  if (L.valt) HB_TRY(tail_values(p, 0));
   if (L.val32) {  // the FP32 copy is rebuilt on next use
     dev_free(L.val32);
     L.val32 = nullptr;
@@ -694,8 +703,11 @@ int hpcg_b200_set_values(hpcg_b200_problem* p, int level, const double* values27
   }
   k_set_values<<<grid_for(c, L.n, 256, 8), 256, 0, c->stream>>>(src, L.new2old, L.val, L.pitch, L.n);
   cudaError_t e = cudaGetLastError();
+  int st = HPCG_B200_OK;
+  if (e == cudaSuccess && L.valt) st = tail_values(p, level);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   cudaFree(tmp);
+  HB_TRY(st);
   if (e != cudaSuccess) {
     set_error("set_values", e);
     return status_of(e);

@@ -643,6 +643,8 @@ int symgs_level(hpcg_b200_problem* p, int l, const double* rhs, double* x, bool 
     if (x_is_zero) HB_CK(cudaMemsetAsync(x, 0, sizeof(double) * L.n, c->stream));
     return gs_natural(c, L, rhs, x);
   }
+  if (!x_is_zero && !dot && !(c->prof && l == 0) && tail_step_ok(p, l) && tail_step(p, l, rhs, x))
+    return HPCG_B200_OK;
   return gs_colour<double, double>(c, L, L.val, rhs, x, x_is_zero, l == 0, dot);
 }
 
@@ -654,6 +656,9 @@ int coarse_vcycle(hpcg_b200_problem* p, bool f32);
 int mg_level(hpcg_b200_problem* p, int l, const double* r, double* x, double* rtz = nullptr) {
   Level& L = p->lev[l];
   Context* c = p->ctx;
+  if (p->symgs_mode == HPCG_B200_SYMGS_COLOUR && !rtz && !(c->prof && l == 0) && l >= tail_first(p, false) &&
+      tail_vcycle(p, l, r, x))
+    return HPCG_B200_OK;
   HB_TRY(symgs_level(p, l, r, x, true));
   if (l + 1 < p->nlev) {
     Level& C = p->lev[l + 1];
@@ -682,6 +687,7 @@ int mg_level(hpcg_b200_problem* p, int l, const double* r, double* x, double* rt
 // the faster way: 32.16 against 32.79 ms per 512^3 iteration, same box.
 // Read after tuning. Measurement knob HPCG_B200_RTZ: "fused" or "pass" forces
 // one way (colour mode with more than one level only).
+// Where the whole V-cycle is one launch (tail.cuh) the CG runs a separate pass.
 bool rtz_fused(const hpcg_b200_problem* P) {
   const Level& L = P->lev[0];
   if (P->symgs_mode != HPCG_B200_SYMGS_COLOUR || P->nlev < 2) return false;
@@ -690,6 +696,7 @@ bool rtz_fused(const hpcg_b200_problem* P) {
     return !e ? 0 : std::strcmp(e, "fused") == 0 ? 1 : std::strcmp(e, "pass") == 0 ? 2 : 0;
   }();
   if (force) return force == 1;
+  if (!P->ctx->prof && tail_first(const_cast<hpcg_b200_problem*>(P), false) == 0) return false;
   return !(L.gs_sched == kBulkCfg && L.colp && L.pack != kPackDiag);
 }
 
@@ -796,6 +803,7 @@ void pick_first(const float (&t)[kColours][kGsConfigs], int (&at)[kColours], int
 
 int autotune(hpcg_b200_problem* P) {
   Context* c = P->ctx;
+  tail_first(P, false);  // may allocate: before any capture
   const char* force = std::getenv("HPCG_B200_CONFIG");
   for (int l = 0; l < P->nlev; ++l) {
     Level& L = P->lev[l];
@@ -954,7 +962,7 @@ int coarse_vcycle(hpcg_b200_problem* p, bool f32) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   HB_CK(cudaStreamIsCapturing(c->stream, &cs));
   if (cs != cudaStreamCaptureStatusNone || p->coarse_graph_failed || !graph_enabled() ||
-      p->symgs_mode != HPCG_B200_SYMGS_COLOUR)
+      p->symgs_mode != HPCG_B200_SYMGS_COLOUR || tail_first(p, f32) <= 1)
     return direct();
   cudaGraphExec_t& ex = p->coarse_graph[f32 ? 1 : 0];
   if (!ex) {
@@ -1308,6 +1316,7 @@ int ensure_f32(hpcg_b200_problem* P) {
 int mg32_level(hpcg_b200_problem* p, int l, const float* r, float* x) {
   Level& L = p->lev[l];
   Context* c = p->ctx;
+  if (!(c->prof && l == 0) && l >= tail_first(p, true) && tail_vcycle(p, l, r, x)) return HPCG_B200_OK;
   HB_TRY((gs_colour<float, float>(c, L, L.val32, r, x, true, l == 0)));
   if (l + 1 < p->nlev) {
     Level& C = p->lev[l + 1];

@@ -1,0 +1,209 @@
+// Host side of the one-launch small end of the V-cycle (tail.cuh): which levels
+// it runs, its shape, and its launch.
+#include <cstdlib>
+
+#include "tail.cuh"
+
+namespace hb {
+
+namespace {
+
+// Largest number of rows a block may have in one colour phase. 256 rows are one
+// chunk of a block's threads; each further chunk adds its own chain, while a
+// phase spread over every SM costs its launch whatever its size. Whole V-cycles
+// measured with the level in and out of this launch, FP64: 256 rows (32^3) 134
+// against 174 us, 400 rows (40x40x32) 169 against 181, 576 rows 194 against 194,
+// 800 rows (40^3) 219 against 186; FP32: 576 rows 183 against 191, 800 rows 195
+// against 189. A lone step also brings x in and its choice is between two
+// launches' worth of set-up: 256 rows 51 against 56 us, 400 rows 66 against 58.
+// Measurement knob: HPCG_B200_TAIL_ROWS.
+int max_rows(bool f32) {
+  static const int forced = [] {
+    const char* e = std::getenv("HPCG_B200_TAIL_ROWS");
+    return e && *e ? std::atoi(e) : 0;
+  }();
+  return forced > 0 ? forced : f32 ? 640 : 448;
+}
+constexpr int kStepRows = 288;
+constexpr int kMaxSmem = 200 * 1024;
+// A level with at most this many rows to a colour stays on one block: its
+// phases then end at the block's own barrier instead of the cluster's.
+constexpr int kOneBlockRows = 128;
+
+int blocks_of(const Level& L) {
+  const int pairs = (L.g.nz + 1) / 2;
+  const int rows = pairs * ((L.g.ny + 1) / 2) * ((L.g.nx + 1) / 2);
+  return rows <= kOneBlockRows ? 1 : std::min(pairs, kTailMaxCluster);
+}
+
+// most z pairs of one block
+int most_pairs(const Level& L, int act) { return ((L.g.nz + 1) / 2 + act - 1) / act; }
+
+// most rows of one block in a phase
+int64_t most_rows(const Level& L, int act) {
+  return (int64_t)most_pairs(L, act) * ((L.g.ny + 1) / 2) * ((L.g.nx + 1) / 2);
+}
+
+int64_t elems_of(const Level& L, int act) {
+  return (int64_t)(2 * most_pairs(L, act) + 2) * TailShape(L.g.nx, L.g.ny).sz;
+}
+// entries of a block's row table: its points
+int64_t rows_of(const Level& L, int act) { return 2ll * most_pairs(L, act) * L.g.ny * L.g.nx; }
+// shared memory of a level
+int64_t bytes_of(const Level& L, int act, bool f32) {
+  return elems_of(L, act) * (f32 ? 4 : 8) + rows_of(L, act) * (int64_t)sizeof(TailRow);
+}
+
+bool level_fits(const Level& L, bool f32) {
+  if (!L.geo || L.next || L.n <= 0) return false;
+  const int act = blocks_of(L);
+  return most_rows(L, act) <= max_rows(f32) && bytes_of(L, act, f32) <= kMaxSmem;
+}
+
+// On unless the environment pins kernel configurations or asks for wavefront
+// sweeps (those are to run), HPCG_B200_TAIL=0 / 1: off / on either way.
+bool wanted() {
+  const char* e = std::getenv("HPCG_B200_TAIL");
+  if (e && *e) return e[0] != '0';
+  const char* a = std::getenv("HPCG_B200_CONFIG");
+  const char* b = std::getenv("HPCG_B200_LEVEL_CONFIG");
+  const char* w = std::getenv("HPCG_B200_WAVE");
+  return !(a && *a) && !(b && *b) && !(w && *w && w[0] != '0');
+}
+
+__global__ void k_tail_values(const double* __restrict__ val, int64_t pitch, double* __restrict__ valt) {
+  const int64_t total = (int64_t)kSlots * pitch;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const int k = (int)(i / pitch);
+    valt[mat_index<double, kTailBlock>(k, i - (int64_t)k * pitch, pitch)] = val[i];
+  }
+}
+
+template <typename T>
+bool launch(hpcg_b200_problem* p, int l, int nlev, const T* rhs, T* x, bool step) {
+  Context* c = p->ctx;
+  TailDesc<T> D;
+  std::memset(&D, 0, sizeof(D));
+  D.nlev = nlev;
+  int cluster = 1;
+  int64_t elems = 0, rows = 0;
+  for (int i = 0; i < nlev; ++i) {
+    const Level& L = p->lev[l + i];
+    TailLevel<T>& t = D.lev[i];
+    if constexpr (sizeof(T) == 4) {
+      t.val = L.val32;
+      t.r = L.r32;
+      t.x = L.x32;
+    } else {
+      t.val = L.valt;
+      t.r = L.r;
+      t.x = L.x;
+    }
+    t.nx = L.g.nx;
+    t.ny = L.g.ny;
+    t.nz = L.g.nz;
+    for (int s = 0; s < kColours; ++s) t.start[s] = L.g.start[s];
+    t.act = blocks_of(L);
+    t.xoff = (int)elems;
+    elems += elems_of(L, t.act);
+    t.toff = (int)rows;
+    rows += rows_of(L, t.act);
+    cluster = std::max(cluster, t.act);
+  }
+  const ColourGrid& g = p->lev[l].g;
+  for (int s = 0; s < kColours; ++s) {
+    D.sweep[s] = g.sweep[s];
+    D.pos[s] = g.pos[s];
+    D.mask[s] = first_mask(g, s);
+  }
+  D.elems = (int)((elems + 1) & ~1ll);  // the row table behind it: 8-byte aligned
+  D.rows = (int)rows;
+  int size = 1;
+  while (size < cluster) size *= 2;
+  auto k = k_tail<T>;
+  const size_t smem = sizeof(T) * (size_t)D.elems + sizeof(TailRow) * (size_t)D.rows;
+  static std::atomic<uint64_t> attr_set{0};
+  const uint64_t bit = 1ull << c->device;
+  if (!(attr_set.load(std::memory_order_acquire) & bit)) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      set_error("k_tail attributes", cudaGetLastError());
+      return false;
+    }
+    attr_set.fetch_or(bit, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(kTailThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k, D, rhs, x, step ? 1 : 0, c->fault);
+  if (e != cudaSuccess) {
+    set_error("k_tail", e);
+    cudaGetLastError();
+    p->tail_first[0] = p->tail_first[1] = p->nlev;
+    return false;
+  }
+  return true;
+}
+
+}  // namespace
+
+int tail_first(hpcg_b200_problem* p, bool f32) {
+  int& first = p->tail_first[f32 ? 1 : 0];
+  if (first >= 0) return first;
+  first = p->nlev;
+  if (!wanted()) return first;
+  int64_t bytes = 256;  // rounding of the table's place
+  int f = p->nlev;
+  for (int l = p->nlev - 1; l >= 0; --l) {
+    const Level& L = p->lev[l];
+    if (!level_fits(L, f32) || (l + 1 < p->nlev && !L.geo_f2c)) break;
+    bytes += bytes_of(L, blocks_of(L), f32);
+    if (bytes > kMaxSmem) break;
+    f = l;
+  }
+  if (!f32)
+    for (int l = f; l < p->nlev; ++l)
+      if (!p->lev[l].valt && tail_values(p, l) != HPCG_B200_OK) return first;  // no memory: the phases run
+  first = f;
+  return first;
+}
+
+// The FP64 values of a small level in the layout tail.cuh reads, built (or,
+// after the values changed, rewritten in place) from the level's own.
+int tail_values(hpcg_b200_problem* p, int l) {
+  Level& L = p->lev[l];
+  Context* c = p->ctx;
+  const int64_t cnt = blocked_entries(L.pitch, kTailBlock);
+  if (!L.valt) {
+    HB_TRY(dev_alloc((void**)&L.valt, sizeof(double) * cnt, &p->bytes));
+    HB_CK(cudaMemsetAsync(L.valt, 0, sizeof(double) * cnt, c->stream));
+  }
+  k_tail_values<<<grid_for(c, (int64_t)kSlots * L.pitch, 256, 8), 256, 0, c->stream>>>(L.val, L.pitch, L.valt);
+  HB_CK(cudaGetLastError());
+  return HPCG_B200_OK;
+}
+
+bool tail_step_ok(hpcg_b200_problem* p, int l) {
+  return tail_first(p, false) <= l && most_rows(p->lev[l], blocks_of(p->lev[l])) <= kStepRows;
+}
+
+bool tail_vcycle(hpcg_b200_problem* p, int l, const double* r, double* x) {
+  return launch<double>(p, l, p->nlev - l, r, x, false);
+}
+bool tail_vcycle(hpcg_b200_problem* p, int l, const float* r, float* x) {
+  return launch<float>(p, l, p->nlev - l, r, x, false);
+}
+bool tail_step(hpcg_b200_problem* p, int l, const double* r, double* x) { return launch<double>(p, l, 1, r, x, true); }
+
+}  // namespace hb
