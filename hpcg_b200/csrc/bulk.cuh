@@ -70,6 +70,9 @@ __host__ __device__ constexpr bool bulk_tensor_tile() {
 // 108; one bulk copy per tile, as the blocked FP32 columns.
 constexpr int kPackBaseWords = 28;
 constexpr int kPackDiag = 3;  // the diagonal form's code
+// The column form of a level whose columns follow from the grid (geo.cuh): a
+// tile is its values alone.
+constexpr int kPackGeo = 4;
 __host__ __device__ constexpr int pack_rec(int w) {
   return kPackBaseWords * 4 + (w == kPackDiag ? kSlots * (kBulkRows / 32) * 4 : kSlots * kBulkRows * w);
 }
@@ -101,7 +104,8 @@ struct BulkShape {
   static constexpr int ring = RING;
   static constexpr int lanes = LANES;
   static constexpr int pack = PW;
-  static constexpr bool packed = PW != 0;
+  static constexpr bool geo = PW == kPackGeo;
+  static constexpr bool packed = PW != 0 && !geo;
   static constexpr int blocks = TB;
   static constexpr int tile_rows = kBulkRows * TB;
   static constexpr int block_threads = kBulkRows * LANES;
@@ -110,7 +114,7 @@ struct BulkShape {
   static constexpr int threads = 32 + groups * group_threads;  // producer warp + consumers
   static constexpr int block_value_bytes = kSlots * kBulkRows * (int)sizeof(T);
   static constexpr int block_col_bytes =
-      PW == 0 ? kSlots * kBulkRows * (int)sizeof(int) : pack_rec(PW < 0 ? 2 : PW);
+      geo ? 0 : PW == 0 ? kSlots * kBulkRows * (int)sizeof(int) : pack_rec(PW < 0 ? 2 : PW);
   static constexpr int value_bytes = block_value_bytes * TB;
   static constexpr int col_bytes = block_col_bytes * TB;
   static_assert(TB == 1 || (TB == 2 && bulk_whole_tile<T>() && PW >= 0 && LANES == 1),
@@ -122,7 +126,7 @@ struct BulkShape {
   static constexpr int smem = stages * stage_bytes + 3 * stages * (int)sizeof(uint64_t) + 128;
   static_assert(smem <= 227 * 1024, "shared memory of one block");
   static_assert(threads <= 1024, "threads of one block");
-  static_assert(PW >= -1 && PW <= kPackDiag, "column form");
+  static_assert(PW >= -1 && PW <= kPackGeo, "column form");
 };
 // The shapes in use: rings of two stages (measured at 512^3: two groups of two
 // stages beat four groups of one for the Gauss-Seidel phases by 8% and tied for
@@ -255,6 +259,8 @@ __device__ __forceinline__ int stage_col(const int* sc, int k, int t, int sink) 
   } else if constexpr (PW == 2) {
     const unsigned o = reinterpret_cast<const unsigned short*>(sc + kPackBaseWords)[k * kBulkRows + t];
     return o == pack_sink(2) ? sink : sc[k] + (int)o;
+  } else if constexpr (PW == kPackGeo) {
+    return 0;  // not from the stage: GeoRow::col
   } else if constexpr (PW == kPackDiag) {
     // the warp's 32 rows share one word of sink bits (a broadcast load)
     const unsigned bits = reinterpret_cast<const unsigned*>(sc + kPackBaseWords)[k * (kBulkRows / 32) + (t >> 5)];
@@ -436,7 +442,9 @@ __device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, R
         // rows q0 .. q0 + kBulkRows of all 27 slots, [slot][row] in shared memory
         if (lane == 0) tma_load_2d(sv, tm_val, (int)ts.q0, 0, &full[s], policy);
       }
-      if constexpr (Shape::packed) {
+      if constexpr (Shape::geo) {
+        // no columns to fetch
+      } else if constexpr (Shape::packed) {
         if (lane == 1) bulk_g2s(sc, ts.rec, rec_bytes, &full[s], policy);
       } else if constexpr (bulk_whole_tile<T>()) {
         if (lane == 1) bulk_g2s(sc, ts.cols, Shape::col_bytes, &full[s], policy);

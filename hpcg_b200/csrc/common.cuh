@@ -187,6 +187,8 @@ struct WaveGeom {
   int start[kColours];  // first row of phase j's colour block
 };
 
+struct GeoGrid;
+
 struct Level {
   ColourGrid g;
   int n = 0;                 // rows
@@ -243,6 +245,9 @@ struct Level {
   // one-launch small levels (tail.cuh) rely on instead of reading them
   bool geo = false;
   bool geo_f2c = false;
+  // the level's colour blocks as the kernels that take the columns from the grid
+  // read them (geo.cuh; host memory), nullptr where they read stored columns
+  GeoGrid* geo_cols = nullptr;
   double* valt = nullptr;  // FP64 values in the layout tail.cuh reads (small levels only, built on first use)
 };
 
@@ -265,6 +270,10 @@ struct hpcg_b200_problem {
   cudaGraphExec_t cg_graph[2];  // instantiated CG loop, [unpreconditioned, preconditioned]
   bool cg_graph_failed;         // capture was refused once: stay with stream launches
   cudaGraphExec_t coarse_graph[2];  // the V-cycle below level 0 as one graph, [FP64, FP32]
+  // the V-cycle on r -> z / r32 -> x32 and the step on r, x as one graph each
+  // (captured on their second use), by CycleKind
+  cudaGraphExec_t cycle_graph[3];
+  unsigned char cycle_uses[3];
   bool coarse_graph_failed;         // its capture was refused once: stream launches
   hb::RankGeom* geom;  // position in a run over several ranks (nullptr: one rank)
   size_t bytes;  // device bytes held
@@ -277,6 +286,8 @@ struct hpcg_b200_problem {
 };
 
 namespace hb {
+
+enum CycleKind : int { kCycleMg = 0, kCycleMg32 = 1, kCycleStep = 2, kCycles = 3 };
 
 // ---- error plumbing ------------------------------------------------------
 void set_error(const char* what, cudaError_t e);

@@ -8,6 +8,7 @@
 
 #include "bulk.cuh"
 #include "common.cuh"
+#include "geo.cuh"
 #include "reduce.cuh"
 #include "rows.cuh"
 
@@ -46,9 +47,11 @@ namespace hb {
 //    see bulk_tiles, k_gs_bulk and k_spmv_bulk.
 constexpr int kConfigs = 8;     // configurations of the SpMV and the restriction
 constexpr int kBulkMvCfg = 7;   // the SpMV through the bulk-copy pipeline (k_spmv_bulk)
-constexpr int kGsConfigs = 11;  // configurations of the Gauss-Seidel phases
+constexpr int kGsConfigs = 13;  // configurations of the Gauss-Seidel phases
+constexpr int kGsFull = 11;     // of which run a phase of all slots (the others: first-sweep phases only)
 constexpr int kTileCfg = 9;     // the tiled configuration
 constexpr int kBulkCfg = 10;    // the bulk-copy pipeline
+constexpr int kGeoCfg = 11;     // and the next: columns from the grid, 1 or 2 rows a thread (k_gs_first_geo)
 // configurations without a row-alignment requirement that run their own kernels
 __host__ __device__ constexpr bool cfg_tiled(int cfg) { return cfg >= kTileCfg; }
 __host__ __device__ constexpr int cfg_sched(int cfg) { return cfg == 2 || cfg == 3 ? kStaged : kPlain; }
@@ -306,15 +309,83 @@ __global__ void k_wait_selftest(unsigned long long limit_ns, unsigned* fault) {
   if (threadIdx.x == 0 && !mbar_wait(&bar, 0, limit_ns)) record_fault(fault, 4);
 }
 
+// First-sweep phase with the columns from the grid (configurations 11 and 12):
+// rows [r0, r1) of the colour block `geo`, the slots of MASK only (their
+// neighbours have been swept, all others multiply a zero). Such a phase reads 13
+// slots on average, so no tile of whole rows is worth staging and its bytes are
+// what bounds it: 8 (FP32 4) a slot here, where the register-pipelined
+// configurations also read the slot's 32-bit column. R rows a thread, 32 apart:
+// every load of a warp is one run, and R rows' loads are in flight; all values
+// of a row are requested before the first gather. The sums are gs_row's.
+template <typename T, typename TR, uint32_t MASK, int R>
+__global__ void __launch_bounds__(kThreads, sizeof(T) * R * __builtin_popcount(MASK) > 128 ? 2 : 4)
+    k_gs_first_geo(const T* __restrict__ val, int64_t pitch, const TR* __restrict__ rhs, T* x, int r0, int r1,
+                   int sink, const __grid_constant__ GeoPhase geo) {
+  const int tile = kThreads * R;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int b0 = r0 + blockIdx.x * tile; b0 < r1; b0 += gridDim.x * tile) {
+    const int q0 = b0 + warp * 32 * R + lane;
+    T a[R][kSlots], d[R], sum[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int q = q0 + 32 * r;
+      if (q < r1) {
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k)
+          if (MASK >> k & 1u) a[r][k] = __ldcs(val + mat_index<T>(k, q, pitch));
+        d[r] = __ldcs(val + mat_index<T>(kDiagSlot, q, pitch));
+        sum[r] = (T)rhs[q];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int q = q0 + 32 * r;
+      if (q < r1) {
+        if (MASK) {
+          const GeoRow g(geo, q);
+          T xv[kSlots];
+#pragma unroll
+          for (int k = 0; k < kSlots; ++k)
+            if (MASK >> k & 1u) xv[k] = __ldg(x + g.col(geo, k, sink));
+#pragma unroll
+          for (int k = 0; k < kSlots; ++k)
+            if (MASK >> k & 1u) sum[r] -= a[r][k] * xv[k];
+        }
+        x[q] = sum[r] / d[r];
+      }
+    }
+  }
+}
+
+// Column of a slot of a row, for each column form of the bulk-copy kernels.
+template <int PW>
+struct ColOf {
+  const int* sc;
+  int t, sink;
+  __device__ __forceinline__ ColOf(const GeoPhase&, int, const int* sc_, int t_, int sink_)
+      : sc(sc_), t(t_), sink(sink_) {}
+  __device__ __forceinline__ int operator()(int k) const { return stage_col<PW>(sc, k, t, sink); }
+};
+template <>
+struct ColOf<kPackGeo> {
+  const GeoPhase& g;
+  GeoRow r;
+  int sink;
+  __device__ __forceinline__ ColOf(const GeoPhase& g_, int q, const int*, int, int sink_)
+      : g(g_), r(g_, q), sink(sink_) {}
+  __device__ __forceinline__ int operator()(int k) const { return r.col(g, k, sink); }
+};
+
 // Gauss-Seidel colour phase over rows [r0, r1) through the pipeline
 // (configuration 10); PW: the level's column form (0: 32-bit columns; 1, 2:
-// the packed record colp with offsets of PW bytes, sink its zero column).
+// the packed record colp with offsets of PW bytes, sink its zero column;
+// kPackGeo: from the grid, geo the phase's colour block).
 template <typename T, typename TR, bool FIRST, int64_t CMASK = -1, bool DOT = false, int PW = 0>
 __global__ void __launch_bounds__(GsShape<T, PW>::threads, 1)
     k_gs_bulk(const T* __restrict__ val, const int* __restrict__ col, int64_t pitch, const TR* __restrict__ rhs,
               T* x, int r0, int r1, uint32_t mask_arg, double* __restrict__ dot, unsigned* fault,
               const __grid_constant__ CUtensorMap tm_val, const __grid_constant__ CUtensorMap tm_col,
-              const unsigned char* __restrict__ colp, int sink) {
+              const unsigned char* __restrict__ colp, int sink, const __grid_constant__ GeoPhase geo) {
   constexpr int TROWS = GsShape<T, PW>::tile_rows;  // 128, or 256 for FP32 tiles of two blocks
   const uint32_t mask = CMASK >= 0 ? (uint32_t)CMASK : mask_arg;
   const int a0 = r0 & ~(TROWS - 1);
@@ -324,6 +395,7 @@ __global__ void __launch_bounds__(GsShape<T, PW>::threads, 1)
       val, col, pitch, ntiles, [&](int tile) { return a0 + (int64_t)tile * TROWS; },
       [&](int64_t q0, const T* sv, const int* sc, int t, auto&&... release) {
         const int64_t q = q0 + t;
+        const ColOf<PW> col_of(geo, (int)q, sc, t, sink);
         if constexpr (sizeof...(release) > 0) {
           // the row's values and columns into registers, the stage back to the producer
           T a[kSlots];
@@ -332,7 +404,7 @@ __global__ void __launch_bounds__(GsShape<T, PW>::threads, 1)
           for (int k = 0; k < kSlots; ++k) {
             if (mask & (1u << k)) {
               a[k] = sv[k * kBulkRows + t];
-              c[k] = stage_col<PW>(sc, k, t, sink);
+              c[k] = col_of(k);
             }
           }
           const T d = sv[kDiagSlot * kBulkRows + t];
@@ -360,7 +432,7 @@ __global__ void __launch_bounds__(GsShape<T, PW>::threads, 1)
           for (int k = 0; k < kSlots; ++k) {
             if (mask & (1u << k)) {
               const T a = sv[k * kBulkRows + t];
-              const T xv = __ldg(x + stage_col<PW>(sc, k, t, sink));
+              const T xv = __ldg(x + col_of(k));
               sum -= a * xv;
               if (k == kDiagSlot) xd = xv;
             }
@@ -559,8 +631,16 @@ __global__ void __launch_bounds__(SpmvShape<T, PW>::threads, 1)
     k_spmv_bulk(ColourGrid g, const T* __restrict__ val, const int* __restrict__ col, int64_t pitch,
                 const T* __restrict__ x, T* __restrict__ y, int n, double* __restrict__ partials, unsigned* fault,
                 const __grid_constant__ CUtensorMap tm_val, const __grid_constant__ CUtensorMap tm_col,
-                const unsigned char* __restrict__ colp, int sink) {
+                const unsigned char* __restrict__ colp, int sink, const __grid_constant__ GeoGrid geo) {
   static_assert(ORDER == 0 || ORDER == 2, "storage or slab order");
+  // the rows of a launch lie in every colour block: their descriptions on chip
+  // (published by the pipeline's first barrier)
+  __shared__ GeoPhase blocks[PW == kPackGeo ? kColours : 1];
+  if constexpr (PW == kPackGeo) {
+    const int* src = reinterpret_cast<const int*>(geo.block);
+    int* dst = reinterpret_cast<int*>(blocks);
+    for (int i = threadIdx.x; i < (int)(sizeof(blocks) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
+  }
   const int ntiles = (n + kBulkRows - 1) / kBulkRows;
   double acc = 0.0;
   bulk_tiles<T, SpmvShape<T, PW>, spmv_early<T>()>(
@@ -570,6 +650,12 @@ __global__ void __launch_bounds__(SpmvShape<T, PW>::threads, 1)
       },
       [&](int64_t q0, const T* sv, const int* sc, int t, auto&&... release) {
         const int64_t q = q0 + t;
+        int at = 0;  // the row's colour block
+        if constexpr (PW == kPackGeo) {
+#pragma unroll
+          for (int s = 1; s < kColours; ++s) at += (int)q >= g.start[s] ? 1 : 0;
+        }
+        const ColOf<PW> col_of(blocks[at], (int)q, sc, t, sink);
         if constexpr (sizeof...(release) > 0) {
           // the row's values and columns into registers, the stage back to the producer
           T a[kSlots];
@@ -577,7 +663,7 @@ __global__ void __launch_bounds__(SpmvShape<T, PW>::threads, 1)
 #pragma unroll
           for (int k = 0; k < kSlots; ++k) {
             a[k] = sv[k * kBulkRows + t];
-            c[k] = stage_col<PW>(sc, k, t, sink);
+            c[k] = col_of(k);
           }
           (release(), ...);
           if (q >= n) return;
@@ -600,14 +686,14 @@ __global__ void __launch_bounds__(SpmvShape<T, PW>::threads, 1)
         // all 27 gathers issued before the first product (the same sum)
         T xv[kSlots];
 #pragma unroll
-        for (int k = 0; k < kSlots; ++k) xv[k] = __ldg(x + stage_col<PW>(sc, k, t, sink));
+        for (int k = 0; k < kSlots; ++k) xv[k] = __ldg(x + col_of(k));
 #pragma unroll
         for (int k = 0; k < kSlots; ++k) sum += sv[k * kBulkRows + t] * xv[k];
         xq = xv[kDiagSlot];
 #else
 #pragma unroll
         for (int k = 0; k < kSlots; ++k) {
-          const T xv = __ldg(x + stage_col<PW>(sc, k, t, sink));
+          const T xv = __ldg(x + col_of(k));
           sum += sv[k * kBulkRows + t] * xv;
           if (k == kDiagSlot) xq = xv;
         }
@@ -667,7 +753,8 @@ __global__ void __launch_bounds__(RestrictShape<T, PW>::threads, 1)
     k_restrict_bulk(const T* __restrict__ val, const int* __restrict__ col, int64_t pitch, const T* __restrict__ rf,
                     const T* __restrict__ xf, const int* __restrict__ tq, T* __restrict__ rc, int f0, int nc,
                     unsigned* fault, const __grid_constant__ CUtensorMap tm_val,
-                    const __grid_constant__ CUtensorMap tm_col, const unsigned char* __restrict__ colp, int sink) {
+                    const __grid_constant__ CUtensorMap tm_col, const unsigned char* __restrict__ colp, int sink,
+                    const __grid_constant__ GeoPhase geo) {
   const int r1 = f0 + nc;
   const int a0 = f0 & ~(kBulkRows - 1);
   const int ntiles = (r1 - a0 + kBulkRows - 1) / kBulkRows;
@@ -675,6 +762,7 @@ __global__ void __launch_bounds__(RestrictShape<T, PW>::threads, 1)
       val, col, pitch, ntiles, [&](int tile) { return a0 + (int64_t)tile * kBulkRows; },
       [&](int64_t q0, const T* sv, const int* sc, int t, auto&&... release) {
         const int64_t f = q0 + t;
+        const ColOf<PW> col_of(geo, (int)f, sc, t, sink);
         if constexpr (sizeof...(release) > 0) {
           // the row's values and columns into registers, the stage back to the producer
           T a[kSlots];
@@ -682,7 +770,7 @@ __global__ void __launch_bounds__(RestrictShape<T, PW>::threads, 1)
 #pragma unroll
           for (int k = 0; k < kSlots; ++k) {
             a[k] = sv[k * kBulkRows + t];
-            c[k] = stage_col<PW>(sc, k, t, sink);
+            c[k] = col_of(k);
           }
           (release(), ...);
           if (f < f0 || f >= r1) return;
@@ -695,7 +783,7 @@ __global__ void __launch_bounds__(RestrictShape<T, PW>::threads, 1)
         if (f < f0 || f >= r1) return;
         T sum = (T)0;
 #pragma unroll
-        for (int k = 0; k < kSlots; ++k) sum += sv[k * kBulkRows + t] * __ldg(xf + stage_col<PW>(sc, k, t, sink));
+        for (int k = 0; k < kSlots; ++k) sum += sv[k * kBulkRows + t] * __ldg(xf + col_of(k));
         rc[tq[f - f0]] = rf[f] - sum;
       },
       fault, tm_val, tm_col, colp);

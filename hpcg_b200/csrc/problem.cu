@@ -11,6 +11,7 @@
 
 #include "bulk.cuh"
 #include "common.cuh"
+#include "geo.cuh"
 #include "shard.cuh"
 
 namespace hb {
@@ -26,11 +27,15 @@ int alloc_n(hpcg_b200_problem* p, T** ptr, int64_t count) {
   return dev_alloc((void**)ptr, sizeof(T) * (size_t)count, &p->bytes);
 }
 
-// Releases the captured coarse V-cycle (0: FP64, 1: FP32); the next stream-run
-// V-cycle captures it again.
+// Releases the captured V-cycles and, FP64, the step (0: FP64, 1: FP32); the
+// next use captures them again.
 void drop_coarse_graph(hpcg_b200_problem* p, int which) {
   if (p->coarse_graph[which]) cudaGraphExecDestroy(p->coarse_graph[which]);
   p->coarse_graph[which] = nullptr;
+  for (int k : {which == 0 ? kCycleMg : kCycleMg32, which == 0 ? kCycleStep : kCycleMg32}) {
+    if (p->cycle_graph[k]) cudaGraphExecDestroy(p->cycle_graph[k]);
+    p->cycle_graph[k] = nullptr;
+  }
 }
 
 hpcg_b200_problem* new_problem(int device, Context* c) {
@@ -355,6 +360,7 @@ int try_pack(hpcg_b200_problem* p, int l) {
 int build_packed(hpcg_b200_problem* p, int l) {
   Level& L = p->lev[l];
   const char* e = std::getenv("HPCG_B200_PACKED");
+  if (L.geo && !(e && *e)) L.geo_cols = new GeoGrid(geo_grid(L.g));  // (a form asked for is the form read)
   if ((e && e[0] == '0') || L.n <= 0) return HPCG_B200_OK;
   const bool only16 = e && std::strcmp(e, "16") == 0;
   const bool from8 = e && std::strcmp(e, "8") == 0;
@@ -375,6 +381,7 @@ int free_problem(hpcg_b200_problem* p) {
     for (void* q : ptrs) dev_free(q);
     delete[] L.wave_start;
     delete L.maps;
+    delete L.geo_cols;
   }
   void* vs[] = {p->b, p->x, p->r, p->z, p->p, p->Ap, p->zprev};
   for (void* q : vs) dev_free(q);
@@ -383,7 +390,7 @@ int free_problem(hpcg_b200_problem* p) {
   free_plans(p);
   for (int i = 0; i < 2; ++i) {
     if (p->cg_graph[i]) cudaGraphExecDestroy(p->cg_graph[i]);
-    if (p->coarse_graph[i]) cudaGraphExecDestroy(p->coarse_graph[i]);
+    drop_coarse_graph(p, i);
   }
   release_accounted(p->bytes);
   p->magic = 0;

@@ -55,6 +55,13 @@ void gs_tile_launch(Context* c, const Level& L, const T* val, const TR* rhs, T* 
   k<<<g, rows, smem, c->stream>>>(val, cols_of<T>(L), L.pitch, rhs, x, r0, r1, mask, dot);
 }
 
+// The sweep position whose rows start at r0.
+inline int sweep_at(const Level& L, int r0) {
+  int s = 0;
+  while (s + 1 < kColours && (L.g.start[s] != r0 || L.g.start[s + 1] == r0)) ++s;
+  return s;
+}
+
 // The bulk-copy pipeline (configuration 10): one block per SM (its shared
 // memory allows no second), at most one per tile; PW: the level's column form
 // (L.pack). false: not launched (FP64 tensor maps unavailable, or refused).
@@ -96,15 +103,17 @@ bool gs_bulk_launch_p(Context* c, const Level& L, const T* val, const TR* rhs, T
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
+  GeoPhase geo{};
+  if constexpr (PW == kPackGeo) geo = L.geo_cols->block[sweep_at(L, r0)];
   cudaError_t e = cudaLaunchKernelEx(&cfg, k, val, cols_of<T>(L), L.pitch, rhs, x, r0, r1, mask, dot, c->fault,
-                                     *tv, *tc, (const unsigned char*)L.colp, sink_of(L));
+                                     *tv, *tc, (const unsigned char*)L.colp, sink_of(L), geo);
   if (e != cudaSuccess && pdl) {
     // refused with the early-launch attribute: record it and launch plainly
     set_error("k_gs_bulk (programmatic dependent launch)", e);
     cudaGetLastError();
     cfg.numAttrs = 0;
     e = cudaLaunchKernelEx(&cfg, k, val, cols_of<T>(L), L.pitch, rhs, x, r0, r1, mask, dot, c->fault, *tv, *tc,
-                           (const unsigned char*)L.colp, sink_of(L));
+                           (const unsigned char*)L.colp, sink_of(L), geo);
   }
   if (e != cudaSuccess) {
     // refused outright (nothing was queued): the caller runs the register kernel instead
@@ -118,6 +127,7 @@ bool gs_bulk_launch_p(Context* c, const Level& L, const T* val, const TR* rhs, T
 template <typename T, typename TR, bool FIRST, int64_t CMASK, bool DOT>
 bool gs_bulk_launch(Context* c, const Level& L, const T* val, const TR* rhs, T* x, int r0, int r1, uint32_t mask,
                     double* dot) {
+  if (L.geo_cols) return gs_bulk_launch_p<T, TR, FIRST, CMASK, DOT, kPackGeo>(c, L, val, rhs, x, r0, r1, mask, dot);
   if (L.pack == kPackDiag)
     return gs_bulk_launch_p<T, TR, FIRST, CMASK, DOT, kPackDiag>(c, L, val, rhs, x, r0, r1, mask, dot);
   if (L.pack == 1) return gs_bulk_launch_p<T, TR, FIRST, CMASK, DOT, 1>(c, L, val, rhs, x, r0, r1, mask, dot);
@@ -178,6 +188,7 @@ void gs_launch(Context* c, const Level& L, const T* val, const TR* rhs, T* x, in
 // on a multiple of R (vector loads); otherwise the scalar configuration 1 runs.
 // Interleaved rows need no alignment.
 inline int usable_cfg(int cfg, int r0) {
+  if (cfg >= kGeoCfg) return kBulkCfg;  // (first-sweep phases only, see gs_first_dispatch)
   return cfg_tiled(cfg) || cfg_interleaved(cfg) || r0 % cfg_rows(cfg) == 0 ? cfg : 1;
 }
 
@@ -215,6 +226,29 @@ void gs_first_const(Context* c, const Level& L, const T* val, const TR* rhs, T* 
   }
 }
 
+// The same on k_gs_first_geo with R rows a thread.
+template <typename T, typename TR, int R, int S>
+void gs_first_geo_at(Context* c, const Level& L, const T* val, const TR* rhs, T* x, int r0, int r1) {
+  if (r1 <= r0) return;
+  auto k = k_gs_first_geo<T, TR, first_mask_default(S), R>;
+  const int64_t units = ((int64_t)r1 - r0 + R - 1) / R;
+  k<<<grid_of(c, k, units), kThreads, 0, c->stream>>>(val, L.pitch, rhs, x, r0, r1, sink_of(L),
+                                                   L.geo_cols->block[S]);
+}
+template <typename T, typename TR, int R>
+void gs_first_geo(Context* c, const Level& L, const T* val, const TR* rhs, T* x, int r0, int r1, int s) {
+  switch (s) {
+    case 0: gs_first_geo_at<T, TR, R, 0>(c, L, val, rhs, x, r0, r1); break;
+    case 1: gs_first_geo_at<T, TR, R, 1>(c, L, val, rhs, x, r0, r1); break;
+    case 2: gs_first_geo_at<T, TR, R, 2>(c, L, val, rhs, x, r0, r1); break;
+    case 3: gs_first_geo_at<T, TR, R, 3>(c, L, val, rhs, x, r0, r1); break;
+    case 4: gs_first_geo_at<T, TR, R, 4>(c, L, val, rhs, x, r0, r1); break;
+    case 5: gs_first_geo_at<T, TR, R, 5>(c, L, val, rhs, x, r0, r1); break;
+    case 6: gs_first_geo_at<T, TR, R, 6>(c, L, val, rhs, x, r0, r1); break;
+    default: gs_first_geo_at<T, TR, R, 7>(c, L, val, rhs, x, r0, r1); break;
+  }
+}
+
 // The first sweep of the default sweep order with compile-time masks; other
 // configurations take the mask at run time.
 template <typename T, typename TR>
@@ -222,6 +256,13 @@ void gs_first_dispatch(Context* c, const Level& L, int cfg, const T* val, const 
                        int s, uint32_t mask) {
   bool default_order = true;
   for (int i = 0; i < kColours; ++i) default_order = default_order && L.g.sweep[i] == kSweepDefault[i];
+  if (cfg >= kGeoCfg && default_order && L.geo_cols) {
+    if (cfg == kGeoCfg)
+      gs_first_geo<T, TR, 1>(c, L, val, rhs, x, r0, r1, s);
+    else
+      gs_first_geo<T, TR, 2>(c, L, val, rhs, x, r0, r1, s);
+    return;
+  }
   const int u = usable_cfg(cfg, r0);
   if (default_order && (u == 0 || u == 1 || u == 4 || u == 5 || u == 7 || u == 8 || cfg_tiled(u))) {
     switch (u) {
@@ -279,8 +320,10 @@ int spmv_bulk_launch(Context* c, const Level& L, const T* val, const T* x, T* y,
   bulk_attr(k, smem, c->device, &attr_set);
   const int64_t tiles = ((int64_t)L.n + kBulkRows - 1) / kBulkRows;
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)c->sms));
+  static const GeoGrid none{};
+  const GeoGrid& geo = PW == kPackGeo ? *L.geo_cols : none;
   k<<<g, Shape::threads, smem, c->stream>>>(L.g, val, cols_of<T>(L), L.pitch, x, y, L.n, partials, c->fault, m->val,
-                                            m->col, (const unsigned char*)L.colp, sink_of(L));
+                                            m->col, (const unsigned char*)L.colp, sink_of(L), geo);
   return g;
 }
 
@@ -304,6 +347,7 @@ int spmv_bulk(Context* c, const Level& L, const T* val, const T* x, T* y, double
     const BulkMaps* m = bulk_maps(L);
     if (!m) return 0;
     if (L.mv_order == 2 && bulk_slab_ok(L)) {
+      if (L.geo_cols) return spmv_bulk_launch<T, DOT, 2, kPackGeo>(c, L, val, x, y, partials, m);
       if (packed_slab_ok(L)) {
         if (L.pack == kPackDiag) return spmv_bulk_launch<T, DOT, 2, kPackDiag>(c, L, val, x, y, partials, m);
         if (L.pack == 1) return spmv_bulk_launch<T, DOT, 2, 1>(c, L, val, x, y, partials, m);
@@ -311,6 +355,7 @@ int spmv_bulk(Context* c, const Level& L, const T* val, const T* x, T* y, double
       }
       return spmv_bulk_launch<T, DOT, 2, 0>(c, L, val, x, y, partials, m);
     }
+    if (L.geo_cols) return spmv_bulk_launch<T, DOT, 0, kPackGeo>(c, L, val, x, y, partials, m);
     if (L.pack == kPackDiag) return spmv_bulk_launch<T, DOT, 0, kPackDiag>(c, L, val, x, y, partials, m);
     if (L.pack == 1) return spmv_bulk_launch<T, DOT, 0, 1>(c, L, val, x, y, partials, m);
     if (L.pack == 2) return spmv_bulk_launch<T, DOT, 0, 2>(c, L, val, x, y, partials, m);
@@ -362,14 +407,17 @@ bool restrict_bulk_p(Context* c, const Level& L, const T* val, const T* rf, cons
   bulk_attr(k, smem, c->device, &attr_set);
   const int64_t tiles = ((int64_t)L.tf_run + nc - (L.tf_run & ~(kBulkRows - 1)) + kBulkRows - 1) / kBulkRows;
   const int g = (int)std::min<int64_t>(tiles, (int64_t)c->sms);
+  GeoPhase geo{};
+  if constexpr (PW == kPackGeo) geo = L.geo_cols->block[sweep_at(L, L.tf_run)];
   k<<<g, Shape::threads, smem, c->stream>>>(val, cols_of<T>(L), L.pitch, rf, xf, L.tq, rc, L.tf_run, nc, c->fault,
-                                            *tv, *tc, (const unsigned char*)L.colp, sink_of(L));
+                                            *tv, *tc, (const unsigned char*)L.colp, sink_of(L), geo);
   return true;
 }
 
 template <typename T>
 bool restrict_bulk(Context* c, const Level& L, const T* val, const T* rf, const T* xf, T* rc, int nc) {
   if (L.tf_run < 0 || nc <= 0) return false;
+  if (L.geo_cols && L.geo_f2c) return restrict_bulk_p<T, kPackGeo>(c, L, val, rf, xf, rc, nc);
   if (L.pack == kPackDiag) return restrict_bulk_p<T, kPackDiag>(c, L, val, rf, xf, rc, nc);
   if (L.pack == 1) return restrict_bulk_p<T, 1>(c, L, val, rf, xf, rc, nc);
   if (L.pack == 2) return restrict_bulk_p<T, 2>(c, L, val, rf, xf, rc, nc);
@@ -697,7 +745,7 @@ bool rtz_fused(const hpcg_b200_problem* P) {
   }();
   if (force) return force == 1;
   if (!P->ctx->prof && tail_first(const_cast<hpcg_b200_problem*>(P), false) == 0) return false;
-  return !(L.gs_sched == kBulkCfg && L.colp && L.pack != kPackDiag);
+  return !(L.gs_sched == kBulkCfg && L.colp && L.pack != kPackDiag && !L.geo_cols);
 }
 
 // Autotuner: per level, times each kernel configuration (load schedule x
@@ -749,7 +797,7 @@ bool level_config_override(int l, int v[6], int* wf, int (&at64)[kColours], int 
       ++s;
     }
   }
-  const int lim[6] = {kGsConfigs, kGsConfigs, kConfigs, 3, kGsConfigs, kGsConfigs};
+  const int lim[6] = {kGsFull, kGsConfigs, kConfigs, 3, kGsFull, kGsConfigs};
   for (int i = 0; i < 6; ++i)
     if (v[i] < 0 || v[i] >= lim[i]) return false;
   if (*s == ',') {
@@ -801,6 +849,46 @@ void pick_first(const float (&t)[kColours][kGsConfigs], int (&at)[kColours], int
   *one = b;
 }
 
+// The configurations of a level whose columns come from the grid: on one rank
+// every kernel has a form that reads the values alone, and which of them is
+// fastest follows from what bounds it, so nothing is timed (timing a new
+// problem's levels took 11-216 ms, and single launches of a few microseconds
+// are not told apart reliably: a step of 96^3 ran in 110 or 181 us from one
+// problem to the next). HPCG_B200_TUNE=1: time them all the same.
+//  - phases of all slots: the bulk-copy pipeline at every size (its early launch
+//    also hides a small phase's start; level 0 of 104^3: 0.44 against 0.54 ms an
+//    iteration with the tuner's pick);
+//  - first-sweep phases: k_gs_first_geo, one row a thread in FP64 (384^3: 1.36 ms a
+//    sweep, two rows 1.47, bulk copies 2.15, the tuner's register mix 1.53), two in
+//    FP32 once the phases leave the L2 (384^3: 0.81 against 0.84 ms; 128^3: 85
+//    against 83 us); the last position reads 26 of 27 slots, so there the bulk
+//    copies win once the matrix comes from memory;
+//  - SpMV: bulk copies, slab order once x no longer fits the L2 beside the matrix
+//    stream (384^3: 1.04 ms; 128^3: 43 us, in storage order 41).
+constexpr int kBeyondL2 = 4 << 20;  // rows: 32 MB a vector, 900 MB of values
+
+bool by_rule(const Level& L) {
+  const char* e = std::getenv("HPCG_B200_TUNE");
+  return L.geo_cols && !(e && *e && e[0] != '0');
+}
+
+void rule_config(Level& L) {
+  const bool large = L.n >= kBeyondL2;
+  L.gs_sched = kBulkCfg;
+  L.gs_first = kGeoCfg;
+  for (int s = 0; s < kColours; ++s) L.gs_first_at[s] = large && s == kColours - 1 ? kBulkCfg : kGeoCfg;
+  L.mv_sched = kBulkMvCfg;
+  L.mv_order = large ? 2 : 0;
+}
+
+void rule_config32(Level& L) {
+  const bool large = L.n >= kBeyondL2;
+  L.gs_sched32 = kBulkCfg;
+  L.gs_first32 = large ? kGeoCfg + 1 : kGeoCfg;
+  for (int s = 0; s < kColours; ++s)
+    L.gs_first32_at[s] = large && s == kColours - 1 ? kBulkCfg : L.gs_first32;
+}
+
 int autotune(hpcg_b200_problem* P) {
   Context* c = P->ctx;
   tail_first(P, false);  // may allocate: before any capture
@@ -823,9 +911,20 @@ int autotune(hpcg_b200_problem* P) {
     }
     if (force && *force) {
       const int f = std::atoi(force);
-      L.gs_sched = L.gs_first = f < 0 ? 0 : f >= kGsConfigs ? kGsConfigs - 1 : f;
+      L.gs_first = f < 0 ? 0 : f >= kGsConfigs ? kGsConfigs - 1 : f;
+      L.gs_sched = std::min(L.gs_first, kGsFull - 1);
       L.mv_sched = f < 0 ? 0 : f >= kConfigs ? kConfigs - 1 : f;
       continue;
+    }
+    if (by_rule(L)) {
+      rule_config(L);
+      const char* fo = std::getenv("HPCG_B200_SPMV_ORDER");
+      if (fo && *fo) L.mv_order = std::atoi(fo);
+      if (wave_force() > 0) {
+        HB_TRY(ensure_wavefront(L));
+        L.wf = L.wf_tpu > 0 ? 1 : 0;
+      }
+      if (wave_force() >= 0) continue;
     }
     double* xs = l == 0 ? P->Ap : L.x;
     double* rs = l == 0 ? P->zprev : L.r;
@@ -858,7 +957,7 @@ int autotune(hpcg_b200_problem* P) {
     const int keep_sched = L.mv_sched, keep_order = L.mv_order;
     for (int rep = 0; rep < 4; ++rep) {
       for (int sched = 0; sched < kGsConfigs; ++sched) {
-        HB_TRY(time_it(t_gs[sched], [&] {
+        if (sched < kGsFull) HB_TRY(time_it(t_gs[sched], [&] {
           gs_dispatch<double, double, false>(c, L, sched, L.val, rs, xs, r0, r1, kAllSlots);
         }));
         // the first-sweep phase of every sweep position (0 to 26 slots)
@@ -947,24 +1046,17 @@ bool graph_enabled() {
 
 int mg32_level(hpcg_b200_problem* p, int l, const float* r, float* x);
 
-// The V-cycle below level 0 (levels 1 .. nlev-1 between the level-0 restriction
-// and prolongation, on the fixed coarse vectors r, x of level 1) for the loops
-// that launch kernel by kernel: captured once as a CUDA graph and launched as
-// one unit, so that its small coarse-level kernels (about 80 of the 117
-// launches of a CG iteration) cost one launch instead of one each. Inside a
-// capture (the CG loop's own graph) and in the natural-order mode the kernels
-// are launched directly; the same kernels either way, so the same bits.
-int coarse_vcycle(hpcg_b200_problem* p, bool f32) {
+// Runs `direct` (launches on c's stream, the same ones every time) as one graph
+// launch once it has been captured into ex; inside a capture, with graphs off
+// or refused, in the natural-order mode and under the launch profiler directly.
+template <typename F>
+int run_captured(hpcg_b200_problem* p, cudaGraphExec_t& ex, F&& direct) {
   Context* c = p->ctx;
-  auto direct = [&]() -> int {
-    return f32 ? mg32_level(p, 1, p->lev[1].r32, p->lev[1].x32) : mg_level(p, 1, p->lev[1].r, p->lev[1].x);
-  };
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   HB_CK(cudaStreamIsCapturing(c->stream, &cs));
-  if (cs != cudaStreamCaptureStatusNone || p->coarse_graph_failed || !graph_enabled() ||
-      p->symgs_mode != HPCG_B200_SYMGS_COLOUR || tail_first(p, f32) <= 1)
+  if (cs != cudaStreamCaptureStatusNone || p->coarse_graph_failed || !graph_enabled() || c->prof ||
+      p->symgs_mode != HPCG_B200_SYMGS_COLOUR)
     return direct();
-  cudaGraphExec_t& ex = p->coarse_graph[f32 ? 1 : 0];
   if (!ex) {
     HB_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     const int st = direct();
@@ -981,6 +1073,40 @@ int coarse_vcycle(hpcg_b200_problem* p, bool f32) {
   }
   HB_CK(cudaGraphLaunch(ex, c->stream));
   return HPCG_B200_OK;
+}
+
+// The V-cycle below level 0 (levels 1 .. nlev-1 between the level-0 restriction
+// and prolongation, on the fixed coarse vectors r, x of level 1) for the loops
+// that launch kernel by kernel: one graph launch instead of one launch for each
+// of its small kernels (a single launch already where tail.cuh runs them all).
+// The same kernels either way, so the same bits.
+int coarse_vcycle(hpcg_b200_problem* p, bool f32) {
+  auto direct = [&]() -> int {
+    return f32 ? mg32_level(p, 1, p->lev[1].r32, p->lev[1].x32) : mg_level(p, 1, p->lev[1].r, p->lev[1].x);
+  };
+  if (tail_first(p, f32) <= 1) return direct();
+  return run_captured(p, p->coarse_graph[f32 ? 1 : 0], direct);
+}
+
+// A V-cycle or step on the problem's own level-0 vectors, as one graph launch
+// from its second use on (a launch costs the host 2-3 us, as long as a small
+// phase runs; a capture costs about what one pass does, so a single use is
+// not captured).
+template <typename F>
+int run_cycle(hpcg_b200_problem* p, CycleKind kind, F&& direct) {
+  if (tail_first(p, kind == kCycleMg32) == 0 && kind != kCycleStep) return direct();  // one launch
+  if (p->cycle_uses[kind] < 1) {
+    ++p->cycle_uses[kind];
+    return direct();
+  }
+  return run_captured(p, p->cycle_graph[kind], direct);
+}
+
+int mg_cycle(hpcg_b200_problem* p) {
+  return run_cycle(p, kCycleMg, [&] { return mg_level(p, 0, p->r, p->z); });
+}
+int mg32_cycle(hpcg_b200_problem* p) {
+  return run_cycle(p, kCycleMg32, [&] { return mg32_level(p, 0, p->lev[0].r32, p->lev[0].x32); });
 }
 
 // One CG iteration (CG.cpp:101-125) with the iteration-aware kernels: the body
@@ -1258,7 +1384,12 @@ int ensure_f32(hpcg_b200_problem* P) {
       const char* force = std::getenv("HPCG_B200_CONFIG");
       if (force && *force) {
         const int f = std::atoi(force);
-        L.gs_sched32 = L.gs_first32 = f < 0 ? 0 : f >= kGsConfigs ? kGsConfigs - 1 : f;
+        L.gs_first32 = f < 0 ? 0 : f >= kGsConfigs ? kGsConfigs - 1 : f;
+        L.gs_sched32 = std::min(L.gs_first32, kGsFull - 1);
+        continue;
+      }
+      if (by_rule(L)) {
+        rule_config32(L);
         continue;
       }
       const int r0 = L.g.start[1], r1 = L.g.start[2];
@@ -1283,7 +1414,7 @@ int ensure_f32(hpcg_b200_problem* P) {
       };
       for (int rep = 0; rep < 4; ++rep) {  // round-robin over the configurations, as in autotune
         for (int cfg = 0; cfg < kGsConfigs; ++cfg) {
-          HB_TRY(time_it(t[cfg], [&] {
+          if (cfg < kGsFull) HB_TRY(time_it(t[cfg], [&] {
             gs_dispatch<float, float, false>(c, L, cfg, L.val32, L.r32, L.x32, r0, r1, kAllSlots);
           }));
           // the first-sweep phase of every sweep position, as in autotune
@@ -1357,7 +1488,7 @@ int run_cg_mixed(hpcg_b200_problem* P, int max_iter, double tol, int* niters, do
     HB_CK(cudaGetLastError());
   }
   for (int k = 1; k <= max_iter && normr / normr0 > tol; ++k) {
-    HB_TRY(mg32_level(P, 0, L.r32, L.x32));
+    HB_TRY(mg32_cycle(P));
     if (k == 1) {
       k_widen_dot<false><<<nb, kThreads, 0, c->stream>>>(n, L.x32, P->r, zc, nullptr, c->partials);
       HB_CK(cudaGetLastError());
@@ -1633,7 +1764,7 @@ int hpcg_b200_symgs(hpcg_b200_problem* p, const double* r, double* x) {
   HB_TRY(load_vector(p, 0, r, p->r));
   HB_TRY(load_vector(p, 0, x, p->x));
   HB_TRY(autotune(p));
-  HB_TRY(symgs_level(p, 0, p->r, p->x, false));
+  HB_TRY(run_cycle(p, kCycleStep, [&] { return symgs_level(p, 0, p->r, p->x, false); }));
   return store_vector(p, 0, p->x, x);
 }
 
@@ -1644,7 +1775,7 @@ int hpcg_b200_mg(hpcg_b200_problem* p, const double* r, double* x) {
   Setter dev(p->device);
   HB_TRY(load_vector(p, 0, r, p->r));
   HB_TRY(autotune(p));
-  HB_TRY(mg_level(p, 0, p->r, p->z));
+  HB_TRY(mg_cycle(p));
   return store_vector(p, 0, p->z, x);
 }
 
@@ -1684,7 +1815,7 @@ int hpcg_b200_mg_f32(hpcg_b200_problem* p, const double* r, double* x) {
   HB_TRY(load_vector(p, 0, r, p->r));
   k_convert<float, double><<<gv, kThreads, 0, c->stream>>>(L.r32, p->r, L.n);
   HB_CK(cudaGetLastError());
-  HB_TRY(mg32_level(p, 0, L.r32, L.x32));
+  HB_TRY(mg32_cycle(p));
   k_convert<double, float><<<gv, kThreads, 0, c->stream>>>(p->z, L.x32, L.n);
   HB_CK(cudaGetLastError());
   return store_vector(p, 0, p->z, x);
