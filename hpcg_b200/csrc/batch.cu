@@ -15,8 +15,10 @@
 #include <vector>
 
 #include "bulk.cuh"
+#include "geo.cuh"
 #include "reduce.cuh"
 #include "rows.cuh"
+#include "tail.cuh"
 
 namespace hb {
 
@@ -41,9 +43,6 @@ struct BGs {
   uint32_t mask;
   int first;
   int prob;
-  const unsigned char* colp;  // the level's packed columns (bulk-copy phases)
-  int pack;                   // their offset width in bytes
-  int sink;                   // the level's zero sink column
 };
 // residual + restriction, and prolongation, of one problem's level
 struct BRes {
@@ -101,61 +100,164 @@ __device__ __forceinline__ void b_gs(const BGs* __restrict__ items, const BTile*
 __global__ void __launch_bounds__(kThreads) k_b_gs(const BGs* __restrict__ items, const BTile* __restrict__ tiles,
                                                    int ntiles, const BScal* __restrict__ sc) { b_gs(items, tiles, ntiles, sc); }
 
-// The batched colour phase through the bulk-copy pipeline (bulk.cuh): every
-// tile is one 128-row block of its problem's blocked FP32 values (val32 of the
-// single-problem path) and one record of its packed columns, so it arrives by
-// two copies; the tiles of problems that have converged are skipped on both
-// sides. Same arithmetic as k_b_gs. The problems' levels may pack their
-// columns with different offset widths: each tile's record states its own.
-// Four consumer groups of one-block tiles.
-#ifndef HB_BATCH_GROUPS
-#define HB_BATCH_GROUPS 4
-#endif
-using BatchShape = BulkShape<float, fit_groups<float, -1>(HB_BATCH_GROUPS, HB_BULK_RING), HB_BULK_RING, 1, -1>;
+// ---- form 1: bulk-copy phases, columns from the grid ---------------------------
+// Every batch member is generated on one rank, so its columns follow from its
+// grids (geo.cuh): a phase's tile is its blocked FP32 values alone (val32 of the
+// single-problem path), and the small levels of all problems are one launch
+// (tail.cuh, a cluster for each problem). The same sums as k_b_gs and its kin.
+
+// one problem's share of a step on one level: a colour phase (rhs -> x), or the
+// residual at the injected rows (rhs, x -> rc through tq)
+struct BGeo {
+  const float* val;
+  const float* rhs;
+  float* x;
+  float* rc;
+  const int* tq;
+  int r0, r1, sink, prob;
+  GeoPhase geo;
+};
+// a tile of rows: everything a producer needs of it in one 32-byte load
+struct alignas(32) BGeoTile {
+  const float* vals;
+  int item, start, prob, pad;
+};
+
+using BatchShape = GsShape<float, kPackGeo>;
+
+// A full-slot phase: the single-problem FP32 phase's pipeline and shape.
 __global__ void __launch_bounds__(BatchShape::threads, 1)
-    k_b_gs_bulk(const BGs* __restrict__ items, const BTile* __restrict__ tiles, int ntiles,
-                const BScal* __restrict__ sc, unsigned* fault) {
-  bulk_tiles_src<float, BatchShape>(
+    k_b_gs_geo(const BGeo* __restrict__ items, const BGeoTile* __restrict__ tiles, int ntiles,
+               const BScal* __restrict__ sc, unsigned* fault) {
+  bulk_tiles_src<float, BatchShape, true>(
       ntiles,
       [&](int t) {
-        const BTile tl = tiles[t];
-        const BGs& it = items[tl.item];
-        return TileSrc<float>{tl.start, it.val + mat_index<float>(0, tl.start, it.pitch),
-                              it.col + mat_index<float>(0, tl.start, it.pitch),
-                              it.colp + (tl.start / kBulkRows) * pack_rec(it.pack), pack_rec(it.pack)};
+        const BGeoTile tl = tiles[t];
+        return TileSrc<float>{tl.start, tl.vals, nullptr, nullptr, 0};
       },
-      [&](int t) { return !sc[items[tiles[t].item].prob].active; },
-      [&](int t, int64_t q0, const float* sv, const int* scol, int row) {
-        const BGs& it = items[tiles[t].item];
-        const int64_t q = q0 + row;
+      [&](int t) { return !sc[tiles[t].prob].active; },
+      [&](int t, int64_t q0, const float* sv, const int*, int row, auto&& release) {
+        const BGeo& it = items[tiles[t].item];
+        const int q = (int)q0 + row;
+        float a[kSlots];
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k) a[k] = sv[k * kBulkRows + row];
+        release();
         if (q < it.r0 || q >= it.r1) return;
-        const uint32_t mask = it.mask;
-        float sum = it.rhs[q];
-        float xd = 0.0f;
-        if (mask == kAllSlots) {  // full-slot phases: the 27 gathers without a test each
+        const GeoRow g(it.geo, q);
+        const float* x = it.x;
+        const int sink = it.sink;
+        float sum = it.rhs[q], xd = 0.0f;
 #pragma unroll
-          for (int k = 0; k < kSlots; ++k) {
-            const float a = sv[k * kBulkRows + row];
-            const float xv = __ldg(it.x + stage_col<-1>(scol, k, row, it.sink));
-            sum -= a * xv;
-            if (k == kDiagSlot) xd = xv;
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < kSlots; ++k) {
-            if (mask & (1u << k)) {
-              const float a = sv[k * kBulkRows + row];
-              const float xv = __ldg(it.x + stage_col<-1>(scol, k, row, it.sink));
-              sum -= a * xv;
-              if (k == kDiagSlot) xd = xv;
-            }
-          }
+        for (int k = 0; k < kSlots; ++k) {
+          const float xv = __ldg(x + g.col(it.geo, k, sink));
+          sum -= a[k] * xv;
+          if (k == kDiagSlot) xd = xv;
         }
-        const float d = sv[kDiagSlot * kBulkRows + row];
-        if (!it.first) sum += xd * d;
-        it.x[q] = sum / d;
+        sum += xd * a[kDiagSlot];
+        it.x[q] = sum / a[kDiagSlot];
       },
       fault, nullptr, nullptr);
+}
+
+// A first-sweep phase (k_gs_first_geo's arithmetic), 256 rows a tile.
+template <uint32_t MASK>
+__global__ void __launch_bounds__(kThreads, __builtin_popcount(MASK) > 16 ? 3 : 4)
+    k_b_first_geo(const BGeo* __restrict__ items, const BGeoTile* __restrict__ tiles, int ntiles,
+                  const BScal* __restrict__ sc) {
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const BGeoTile tl = tiles[t];
+    if (!sc[tl.prob].active) continue;
+    const BGeo& it = items[tl.item];
+    const int q = tl.start + threadIdx.x;
+    if (q >= it.r1) continue;
+    float a[kSlots];
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k)
+      if (MASK >> k & 1u) a[k] = __ldcs(it.val + mat_index<float>(k, q, 0));
+    const float d = __ldcs(it.val + mat_index<float>(kDiagSlot, q, 0));
+    float sum = it.rhs[q];
+    if (MASK) {
+      const GeoRow g(it.geo, q);
+      float xv[kSlots];
+#pragma unroll
+      for (int k = 0; k < kSlots; ++k)
+        if (MASK >> k & 1u) xv[k] = __ldg(it.x + g.col(it.geo, k, it.sink));
+#pragma unroll
+      for (int k = 0; k < kSlots; ++k)
+        if (MASK >> k & 1u) sum -= a[k] * xv[k];
+    }
+    it.x[q] = sum / d;
+  }
+}
+
+// Residual at the injected rows (k_b_restrict's arithmetic): rows r0 .. r1 are
+// the all-even points, tq their coarse rows.
+__global__ void __launch_bounds__(kThreads, 3)
+    k_b_restrict_geo(const BGeo* __restrict__ items, const BGeoTile* __restrict__ tiles, int ntiles,
+                     const BScal* __restrict__ sc) {
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const BGeoTile tl = tiles[t];
+    if (!sc[tl.prob].active) continue;
+    const BGeo& it = items[tl.item];
+    const int q = tl.start + threadIdx.x;
+    if (q >= it.r1) continue;
+    float a[kSlots];
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k) a[k] = __ldcs(it.val + mat_index<float>(k, q, 0));
+    const GeoRow g(it.geo, q);
+    float sum = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k) sum += a[k] * __ldg(it.x + g.col(it.geo, k, it.sink));
+    it.rc[it.tq[q - it.r0]] = it.rhs[q] - sum;
+  }
+}
+
+// The small levels of every active problem: cluster p of the grid runs problem
+// p's (tail.cuh).
+__global__ void __launch_bounds__(kTailThreads, 2)
+    k_b_tail(const TailDesc<float>* __restrict__ descs, const BScal* __restrict__ sc, unsigned* fault) {
+  __shared__ TailDesc<float> D;
+  const int p = (int)(blockIdx.x / cluster_blocks());
+  if (!sc[p].active || descs[p].nlev == 0) return;  // the whole cluster
+  const int* src = reinterpret_cast<const int*>(&descs[p]);
+  for (int i = threadIdx.x; i < (int)(sizeof(D) / sizeof(int)); i += kTailThreads) reinterpret_cast<int*>(&D)[i] = src[i];
+  __syncthreads();
+  tail_run<float>(D, D.lev[0].r, D.lev[0].x, false, fault);
+}
+
+// y = A x and partials of x'y per tile (b_spmv's arithmetic), columns from the grid.
+__global__ void __launch_bounds__(kThreads, 2)
+    k_b_spmv_geo(const BVec* __restrict__ v, const GeoGrid* __restrict__ grids, const BTile* __restrict__ tiles,
+                 int ntiles, const BScal* __restrict__ sc, double* __restrict__ partials) {
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const BTile tl = tiles[t];
+    const BVec& it = v[tl.item];
+    double acc = 0.0;
+    const int q = tl.start + threadIdx.x;
+    if (sc[tl.item].active && q < it.n) {
+      double a[kSlots];
+#pragma unroll
+      for (int k = 0; k < kSlots; ++k) a[k] = __ldcs(it.val + k * it.pitch + q);
+      const GeoGrid& G = grids[tl.item];
+      int at = 0;
+#pragma unroll
+      for (int s = 1; s < kColours; ++s) at += q >= G.block[s].start ? 1 : 0;
+      const GeoPhase& b = G.block[at];
+      const GeoRow g(b, q);
+      double sum = 0.0, xq = 0.0;
+#pragma unroll
+      for (int k = 0; k < kSlots; ++k) {
+        const double xv = __ldg(it.p + g.col(b, k, it.n));
+        sum += a[k] * xv;
+        if (k == kDiagSlot) xq = xv;
+      }
+      it.Ap[q] = sum;
+      acc = xq * sum;
+    }
+    const double s = block_sum(acc);
+    if (threadIdx.x == 0) partials[t] = s;
+  }
 }
 
 // rc = (rf - A xf) at the injected rows (ComputeMG_ref.cpp:49-51, sorted pairs)
@@ -567,8 +669,14 @@ struct Step {
   int item_off;  // first item of the step (tiles index the whole item array)
   int tile_off;  // first tile of the step
   int ntiles;
-  int btile_off = 0;  // GS phases: the step's 128-row tiles for k_b_gs_bulk
-  int bntiles = 0;
+};
+
+// A step of form 1's V-cycle.
+struct GeoStep {
+  enum Kind { kFull, kFirst, kRestrict, kProlong, kTail } kind;
+  int s;         // kFirst: sweep position
+  int tile_off;  // first tile
+  int ntiles;
 };
 
 }  // namespace
@@ -584,14 +692,21 @@ struct hpcg_b200_batch {
   hb::BGs* gs_items;
   hb::BRes* res_items;
   hb::BTile* tiles;
-  hb::BGs* gs_bitems;  // the GS items on the blocked FP32 copies (bulk-copy phases)
-  hb::BTile* btiles;   // their 128-row tiles
-  bool bulk;           // GS phases on k_b_gs_bulk (chosen by timing at creation)
-  bool persist;        // the whole iteration as one cooperative launch (k_b_iteration), chosen likewise
+  bool bulk;           // form 1
+  bool persist;        // form 2: the whole iteration as one cooperative launch (k_b_iteration)
+  // form 1's work lists (device) and steps
+  hb::BGeo* geo_items;
+  hb::BGeoTile* geo_tiles;
+  hb::BRes* prolong_items;
+  hb::BTile* prolong_tiles;
+  hb::GeoGrid* grids;            // [m] level 0
+  hb::TailDesc<float>* descs;    // [m] the small levels (nlev 0: none)
+  std::vector<hb::GeoStep> geo_steps;
+  int tail_cluster;              // blocks of a cluster
+  size_t tail_smem;
   int persist_grid;    // its blocks: as many as the SMs hold at once
   hb::DStep* dsteps;   // the V-cycle's steps for k_b_iteration
   hb::BBar* bar;       // its grid barrier
-  bool packed;         // every level of every problem has packed columns (k_b_gs_bulk reads them)
   std::vector<hb::Step> steps;
   hb::BVec* vec;
   hb::BTile* vtiles;  // row tiles of every problem's level 0
@@ -630,21 +745,14 @@ void tiles_of(std::vector<BTile>& tiles, int item, int r0, int r1) {
   for (int s = r0; s < r1; s += kTile) tiles.push_back({item, s});
 }
 
-// 128-row tiles of the bulk-copy phase: blocks of the blocked FP32 copy that
-// hold rows of [r0, r1)
-void bulk_tiles_of(std::vector<BTile>& tiles, int item, int r0, int r1) {
-  for (int s = r0 & ~(kBulkRows - 1); s < r1; s += kBulkRows) tiles.push_back({item, s});
-}
-
 // The V-cycle of every problem as one step sequence (ComputeMG_ref.cpp:39-63
 // with the colour sweeps of the single-problem path): level l pre-smooth
 // (forward from x = 0, backward without the last colour), restriction,
 // recursion, prolongation, post-smooth; the coarsest level one symmetric sweep.
 void build_vcycle(hpcg_b200_batch* B, int l, std::vector<BGs>& gs, std::vector<BRes>& res,
-                  std::vector<BTile>& tiles, std::vector<BGs>& gsb, std::vector<BTile>& btiles) {
+                  std::vector<BTile>& tiles) {
   auto phase = [&](int s, bool first) {
     Step st{0, (int)gs.size(), (int)tiles.size(), 0};
-    st.btile_off = (int)btiles.size();
     for (int p = 0; p < B->m; ++p) {
       const Level& L = B->probs[p]->lev[l];
       const int item = (int)gs.size();
@@ -659,23 +767,10 @@ void build_vcycle(hpcg_b200_batch* B, int l, std::vector<BGs>& gs, std::vector<B
       it.mask = first ? first_mask(L.g, s) : kAllSlots;
       it.first = first ? 1 : 0;
       it.prob = p;
-      it.colp = nullptr;
-      it.pack = 0;
-      it.sink = 0;
       gs.push_back(it);
       tiles_of(tiles, item, it.r0, it.r1);
-      BGs bit = it;  // the same phase on the blocked copies (item index = gs index)
-      bit.val = L.val32;
-      bit.col = L.col32;
-      bit.colp = L.colp;
-      bit.pack = L.pack;
-      bit.sink = sink_of(L);
-      if (!L.colp) B->packed = false;  // the bulk-copy phases need packed columns
-      gsb.push_back(bit);
-      bulk_tiles_of(btiles, item, it.r0, it.r1);
     }
     st.ntiles = (int)tiles.size() - st.tile_off;
-    st.bntiles = (int)btiles.size() - st.btile_off;
     B->steps.push_back(st);
   };
   auto sweep = [&](bool first) {
@@ -714,9 +809,85 @@ void build_vcycle(hpcg_b200_batch* B, int l, std::vector<BGs>& gs, std::vector<B
   sweep(true);
   if (l + 1 < 4) {
     transfer(1);
-    build_vcycle(B, l + 1, gs, res, tiles, gsb, btiles);
+    build_vcycle(B, l + 1, gs, res, tiles);
     transfer(2);
     sweep(false);
+  }
+}
+
+// Form 1's V-cycle: as build_vcycle, problem p taking part in the steps of the
+// levels above tail_first; the rest is one launch.
+struct GeoLists {
+  std::vector<BGeo> items;
+  std::vector<BGeoTile> tiles;
+  std::vector<BRes> res;
+  std::vector<BTile> rtiles;
+};
+void build_geo(hpcg_b200_batch* B, int l, GeoLists& W) {
+  const int m = B->m;
+  std::vector<int> in;
+  for (int p = 0; p < m; ++p)
+    if (l < kMaxLevels && tail_first(B->probs[p], true) > l) in.push_back(p);
+  if (in.empty() || l >= kMaxLevels) {  // the others' levels are done above: now the small ones of all
+    bool any = false;
+    for (int p = 0; p < m; ++p) any = any || tail_first(B->probs[p], true) < B->probs[p]->nlev;
+    if (any) B->geo_steps.push_back(GeoStep{GeoStep::kTail, 0, 0, 0});
+    return;
+  }
+  auto step = [&](GeoStep::Kind kind, int s, int rows) {
+    GeoStep st{kind, s, (int)W.tiles.size(), 0};
+    for (int p : in) {
+      const Level& L = B->probs[p]->lev[l];
+      const int item = (int)W.items.size();
+      BGeo it;
+      it.val = L.val32;
+      it.rhs = L.r32;
+      it.x = L.x32;
+      it.rc = kind == GeoStep::kRestrict ? B->probs[p]->lev[l + 1].r32 : nullptr;
+      it.tq = L.tq;
+      it.r0 = L.g.start[s];
+      it.r1 = L.g.start[s + 1];
+      it.sink = sink_of(L);
+      it.prob = p;
+      it.geo = L.geo_cols->block[s];
+      W.items.push_back(it);
+      // whole-block tiles for the copies, from the first row for the others
+      const int first = kind == GeoStep::kFull ? it.r0 / rows * rows : it.r0;
+      for (int q = first; q < it.r1; q += rows)
+        W.tiles.push_back(BGeoTile{L.val32 + mat_index<float>(0, q, 0), item, q, p, 0});
+    }
+    st.ntiles = (int)W.tiles.size() - st.tile_off;
+    B->geo_steps.push_back(st);
+  };
+  auto sweep = [&](bool first) {
+    for (int s = 0; s < kColours; ++s)
+      step(first ? GeoStep::kFirst : GeoStep::kFull, s, first ? kTile : BatchShape::tile_rows);
+    for (int s = kColours - 2; s >= 0; --s) step(GeoStep::kFull, s, BatchShape::tile_rows);
+  };
+  sweep(true);
+  if (l + 1 < kMaxLevels) {
+    step(GeoStep::kRestrict, kColours - 1, kTile);
+    build_geo(B, l + 1, W);
+    GeoStep st{GeoStep::kProlong, 0, (int)W.rtiles.size(), 0};
+    for (int p : in) {
+      const Level& L = B->probs[p]->lev[l];
+      const Level& C = B->probs[p]->lev[l + 1];
+      const int item = (int)W.res.size();
+      BRes it{};
+      it.tf = L.tf;
+      it.tq = L.tq;
+      it.nc = C.n;
+      it.prob = p;
+      it.rf = C.x32;
+      it.rc = L.x32;
+      W.res.push_back(it);
+      tiles_of(W.rtiles, item, 0, it.nc);
+    }
+    st.ntiles = (int)W.rtiles.size() - st.tile_off;
+    B->geo_steps.push_back(st);
+    sweep(false);
+  } else {
+    build_geo(B, l + 1, W);
   }
 }
 
@@ -729,19 +900,78 @@ int launch_step(hpcg_b200_batch* B, const Step& s) {
   Context* c = B->ctx;
   const int g = grid_tiles(c, s.ntiles);
   // tiles hold indices into the whole item array, so the items go in unshifted
-  if (s.kind == 0 && B->bulk) {
-    using Sh = BatchShape;
-    static std::atomic<uint64_t> attr_set{0};  // devices on which the shared-memory size is enabled
-    bulk_attr(k_b_gs_bulk, Sh::smem, c->device, &attr_set);
-    const int gb = s.bntiles < c->sms ? (s.bntiles < 1 ? 1 : s.bntiles) : c->sms;
-    k_b_gs_bulk<<<gb, Sh::threads, Sh::smem, c->stream>>>(B->gs_bitems, B->btiles + s.btile_off, s.bntiles, B->sc,
-                                                          c->fault);
-  } else if (s.kind == 0)
+  if (s.kind == 0)
     k_b_gs<<<g, kThreads, 0, c->stream>>>(B->gs_items, B->tiles + s.tile_off, s.ntiles, B->sc);
   else if (s.kind == 1)
     k_b_restrict<<<g, kThreads, 0, c->stream>>>(B->res_items, B->tiles + s.tile_off, s.ntiles, B->sc);
   else
     k_b_prolong<<<g, kThreads, 0, c->stream>>>(B->res_items, B->tiles + s.tile_off, s.ntiles, B->sc);
+  HB_CK(cudaGetLastError());
+  return HPCG_B200_OK;
+}
+
+template <int S>
+void launch_first_geo(hpcg_b200_batch* B, const GeoStep& st) {
+  Context* c = B->ctx;
+  k_b_first_geo<first_mask_default(S)><<<grid_tiles(c, st.ntiles), kThreads, 0, c->stream>>>(
+      B->geo_items, B->geo_tiles + st.tile_off, st.ntiles, B->sc);
+}
+
+int launch_geo_step(hpcg_b200_batch* B, const GeoStep& st) {
+  Context* c = B->ctx;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const BGeoTile* tiles = B->geo_tiles + st.tile_off;
+  switch (st.kind) {
+    case GeoStep::kFull: {
+      static std::atomic<uint64_t> attr_set{0};  // devices on which the shared-memory size is enabled
+      bulk_attr(k_b_gs_geo, BatchShape::smem, c->device, &attr_set);
+      cfg.gridDim = dim3(std::max(1, std::min(st.ntiles, c->sms)));
+      cfg.blockDim = dim3(BatchShape::threads);
+      cfg.dynamicSmemBytes = BatchShape::smem;
+      // early launch: the producer reads values and, for the tiles to skip, the
+      // convergence flags, which are written before a plainly launched kernel
+      // (a first-sweep phase, a prolongation) of every V-cycle
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      HB_CK(cudaLaunchKernelEx(&cfg, k_b_gs_geo, (const BGeo*)B->geo_items, tiles, st.ntiles, (const BScal*)B->sc,
+                               c->fault));
+      return HPCG_B200_OK;
+    }
+    case GeoStep::kFirst:
+      switch (st.s) {
+        case 0: launch_first_geo<0>(B, st); break;
+        case 1: launch_first_geo<1>(B, st); break;
+        case 2: launch_first_geo<2>(B, st); break;
+        case 3: launch_first_geo<3>(B, st); break;
+        case 4: launch_first_geo<4>(B, st); break;
+        case 5: launch_first_geo<5>(B, st); break;
+        case 6: launch_first_geo<6>(B, st); break;
+        default: launch_first_geo<7>(B, st); break;
+      }
+      break;
+    case GeoStep::kRestrict:
+      k_b_restrict_geo<<<grid_tiles(c, st.ntiles), kThreads, 0, c->stream>>>(B->geo_items, tiles, st.ntiles, B->sc);
+      break;
+    case GeoStep::kProlong:
+      k_b_prolong<<<grid_tiles(c, st.ntiles), kThreads, 0, c->stream>>>(
+          B->prolong_items, B->prolong_tiles + st.tile_off, st.ntiles, B->sc);
+      break;
+    case GeoStep::kTail:
+      cfg.gridDim = dim3(B->m * B->tail_cluster);
+      cfg.blockDim = dim3(kTailThreads);
+      cfg.dynamicSmemBytes = B->tail_smem;
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = B->tail_cluster;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      HB_CK(cudaLaunchKernelEx(&cfg, k_b_tail, (const TailDesc<float>*)B->descs, (const BScal*)B->sc, c->fault));
+      return HPCG_B200_OK;
+  }
   HB_CK(cudaGetLastError());
   return HPCG_B200_OK;
 }
@@ -758,12 +988,18 @@ int iteration(hpcg_b200_batch* B) {
   const int gv = grid_tiles(c, B->nvt);
   k_b_to32<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc);
   HB_CK(cudaGetLastError());
-  for (const Step& s : B->steps) HB_TRY(launch_step(B, s));
+  if (B->bulk)
+    for (const GeoStep& s : B->geo_steps) HB_TRY(launch_geo_step(B, s));
+  else
+    for (const Step& s : B->steps) HB_TRY(launch_step(B, s));
   k_b_to64_dots<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->partials);
   HB_CK(cudaGetLastError());
   HB_TRY(finalize_b(B, kBRtz));
   k_b_update_p<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->ctl);
-  k_b_spmv<true><<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, 1, B->sc, B->partials);
+  if (B->bulk)
+    k_b_spmv_geo<<<gv, kThreads, 0, c->stream>>>(B->vec, B->grids, B->vtiles, B->nvt, B->sc, B->partials);
+  else
+    k_b_spmv<true><<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, 1, B->sc, B->partials);
   HB_CK(cudaGetLastError());
   HB_TRY(finalize_b(B, kBPap));
   k_b_update_xr<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->partials);
@@ -869,68 +1105,79 @@ int build_graph(hpcg_b200_batch* B) {
   return st;
 }
 
-// The form of an iteration: one launch per step with the colour phases on the
-// register kernel (k_b_gs) or on the bulk-copy kernel (k_b_gs_bulk, every
-// level packed), or the whole iteration as one cooperative launch
-// (k_b_iteration, register phases). The fastest V-cycle (all problems active,
-// three rounds each way, round-robin), or HPCG_B200_BATCH_PERSIST (1: one
-// launch) / HPCG_B200_BATCH_BULK (one launch per step; 1: bulk-copy phases).
-// Every V-cycle starts its sweeps from the right-hand side alone, so the work
-// vectors it leaves behind are rewritten by the next solve.
+// The form of an iteration (hpcg_b200_batch_form): 1, the bulk-copy phases with
+// columns from the grid and the small levels in one launch, where every level's
+// columns follow from its grid (every batch unless HPCG_B200_PACKED asks for
+// stored ones), else 0, one launch per step on the register kernels.
+// HPCG_B200_BATCH_PERSIST=1: 2, the whole iteration as one cooperative launch;
+// HPCG_B200_BATCH_BULK=0 (or PERSIST=0 without BULK=1): 0. Sixteen problems of
+// sides 32 to 128: form 1 takes BATCH_FORM1 ms to 1e-9, form 0 105.
 int choose_form(hpcg_b200_batch* B) {
   const char* fp = std::getenv("HPCG_B200_BATCH_PERSIST");
   const char* fb = std::getenv("HPCG_B200_BATCH_BULK");
-  if (fp && *fp) {
-    B->persist = std::atoi(fp) != 0 && B->persist_grid > 0;
-    B->bulk = !B->persist && B->packed && fb && *fb && std::atoi(fb) != 0;
-    return HPCG_B200_OK;
-  }
-  if (fb && *fb) {
-    B->persist = false;
-    B->bulk = B->packed && std::atoi(fb) != 0;
-    return HPCG_B200_OK;
-  }
-  Context* c = B->ctx;
-  std::vector<BScal> on(B->m);
-  for (BScal& x : on) {
-    std::memset(&x, 0, sizeof(x));
-    x.active = 1;
-  }
-  HB_CK(cudaMemcpy(B->sc, on.data(), sizeof(BScal) * B->m, cudaMemcpyHostToDevice));
-  cudaEvent_t e0, e1;
-  HB_CK(cudaEventCreate(&e0));
-  HB_CK(cudaEventCreate(&e1));
-  float best[3] = {1e30f, 1e30f, 1e30f};
-  const bool can[3] = {true, B->packed, B->persist_grid > 0};
-  int st = HPCG_B200_OK;
-  for (int rep = 0; rep < 3 && st == HPCG_B200_OK; ++rep) {
-    for (int f = 0; f < 3 && st == HPCG_B200_OK; ++f) {
-      if (!can[f]) continue;
-      B->bulk = f == 1;
-      if (cudaEventRecord(e0, c->stream) != cudaSuccess) st = HPCG_B200_ERR_CUDA;
-      if (f == 2) {
-        if (st == HPCG_B200_OK) st = launch_iteration(B, true);
-      } else {
-        for (const Step& s : B->steps)
-          if (st == HPCG_B200_OK) st = launch_step(B, s);
-      }
-      if (st == HPCG_B200_OK && cudaEventRecord(e1, c->stream) != cudaSuccess) st = HPCG_B200_ERR_CUDA;
-      if (st == HPCG_B200_OK) st = stream_sync(c);
-      float ms = 0.f;
-      if (st == HPCG_B200_OK && cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) st = HPCG_B200_ERR_CUDA;
-      if (st == HPCG_B200_OK && ms < best[f]) best[f] = ms;
+  bool geo = true;
+  for (hpcg_b200_problem* p : B->probs)
+    for (int l = 0; l < p->nlev; ++l) geo = geo && p->lev[l].geo_cols && p->lev[l].tf_run >= (l + 1 < p->nlev ? 0 : -1);
+  const bool want = fb && *fb ? std::atoi(fb) != 0 : !(fp && *fp);
+  B->persist = fp && *fp && std::atoi(fp) != 0 && B->persist_grid > 0;
+  B->bulk = !B->persist && geo && want;
+  return HPCG_B200_OK;
+}
+
+// Form 1's work lists.
+int build_form1(hpcg_b200_batch* B) {
+  GeoLists W;
+  build_geo(B, 0, W);
+  std::vector<TailDesc<float>> descs(B->m);
+  std::vector<GeoGrid> grids;
+  B->tail_cluster = 1;
+  B->tail_smem = 0;
+  for (int p = 0; p < B->m; ++p) {
+    hpcg_b200_problem* P = B->probs[p];
+    grids.push_back(*P->lev[0].geo_cols);
+    std::memset(&descs[p], 0, sizeof(descs[p]));
+    const int l = tail_first(P, true);
+    if (l < P->nlev) {
+      size_t smem = 0;
+      B->tail_cluster = std::max(B->tail_cluster, tail_desc(P, l, P->nlev - l, &descs[p], &smem));
+      B->tail_smem = std::max(B->tail_smem, smem);
     }
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  HB_TRY(st);
-  int f = 0;
-  for (int i = 1; i < 3; ++i)
-    if (best[i] < best[f]) f = i;
-  B->bulk = f == 1;
-  B->persist = f == 2;
-  HB_CK(cudaMemset(B->sc, 0, sizeof(BScal) * B->m));
-  return HPCG_B200_OK;
+  HB_TRY(tail_attributes((const void*)k_b_tail, B->tail_smem));
+  HB_TRY(alloc_copy(B, (void**)&B->geo_items, W.items.data(), sizeof(BGeo) * W.items.size()));
+  HB_TRY(alloc_copy(B, (void**)&B->geo_tiles, W.tiles.data(), sizeof(BGeoTile) * W.tiles.size()));
+  HB_TRY(alloc_copy(B, (void**)&B->prolong_items, W.res.data(), sizeof(BRes) * W.res.size()));
+  HB_TRY(alloc_copy(B, (void**)&B->prolong_tiles, W.rtiles.data(), sizeof(BTile) * W.rtiles.size()));
+  HB_TRY(alloc_copy(B, (void**)&B->grids, grids.data(), sizeof(GeoGrid) * grids.size()));
+  return alloc_copy(B, (void**)&B->descs, descs.data(), sizeof(TailDesc<float>) * descs.size());
+}
+
+// Forms 0 and 2: slot-major FP32 values and the work lists of the register kernels.
+int build_register_forms(hpcg_b200_batch* B) {
+  Context* c = B->ctx;
+  for (hpcg_b200_problem* p : B->probs)
+    for (int l = 0; l < kMaxLevels; ++l) {
+      float* v = nullptr;
+      if (l < p->nlev) {
+        const int64_t cnt = (int64_t)kSlots * p->lev[l].pitch;
+        HB_TRY(dev_alloc((void**)&v, sizeof(float) * cnt, &B->bytes));
+        B->val32.push_back(v);
+        k_narrow<<<grid_for(c, cnt, kThreads, 8), kThreads, 0, c->stream>>>(v, p->lev[l].val, cnt);
+        HB_CK(cudaGetLastError());
+      } else {
+        B->val32.push_back(v);
+      }
+    }
+  std::vector<BGs> gs;
+  std::vector<BRes> res;
+  std::vector<BTile> tiles;
+  build_vcycle(B, 0, gs, res, tiles);
+  HB_TRY(alloc_copy(B, (void**)&B->gs_items, gs.data(), sizeof(BGs) * gs.size()));
+  if (!res.empty()) HB_TRY(alloc_copy(B, (void**)&B->res_items, res.data(), sizeof(BRes) * res.size()));
+  HB_TRY(alloc_copy(B, (void**)&B->tiles, tiles.data(), sizeof(BTile) * tiles.size()));
+  std::vector<DStep> ds;
+  for (const Step& x : B->steps) ds.push_back(DStep{x.kind, x.tile_off, x.ntiles});
+  return alloc_copy(B, (void**)&B->dsteps, ds.data(), sizeof(DStep) * ds.size());
 }
 
 void destroy(hpcg_b200_batch* B) {
@@ -938,8 +1185,8 @@ void destroy(hpcg_b200_batch* B) {
   cudaSetDevice(B->device);
   if (B->ctx) cudaStreamSynchronize(B->ctx->stream);
   if (B->graph) cudaGraphExecDestroy(B->graph);
-  void* v[] = {B->gs_items, B->res_items, B->tiles, B->gs_bitems, B->btiles, B->vec, B->vtiles, B->vrange,
-               B->partials, B->sc, B->ctl, B->dsteps, B->bar};
+  void* v[] = {B->gs_items, B->res_items, B->tiles, B->geo_items, B->geo_tiles, B->prolong_items, B->prolong_tiles,
+               B->grids, B->descs, B->vec, B->vtiles, B->vrange, B->partials, B->sc, B->ctl, B->dsteps, B->bar};
   for (void* q : v) cudaFree(q);
   for (float* q : B->val32) cudaFree(q);
   if (B->sc_host) cudaFreeHost(B->sc_host);
@@ -972,7 +1219,8 @@ int hpcg_b200_batch_create(int count, const int* nx, const int* ny, const int* n
   B->ctx = c;
   B->m = count;
   B->gs_items = nullptr; B->res_items = nullptr; B->tiles = nullptr; B->vec = nullptr; B->vtiles = nullptr;
-  B->gs_bitems = nullptr; B->btiles = nullptr; B->bulk = false; B->packed = true;
+  B->geo_items = nullptr; B->geo_tiles = nullptr; B->prolong_items = nullptr; B->prolong_tiles = nullptr;
+  B->grids = nullptr; B->descs = nullptr; B->bulk = false; B->tail_cluster = 1; B->tail_smem = 0;
   B->persist = false; B->persist_grid = 0; B->dsteps = nullptr; B->bar = nullptr;
   B->vrange = nullptr; B->partials = nullptr; B->sc = nullptr; B->sc_host = nullptr; B->ctl = nullptr;
   B->bytes = 0;
@@ -986,25 +1234,8 @@ int hpcg_b200_batch_create(int count, const int* nx, const int* ny, const int* n
       B->probs.push_back(p);
       st = prepare_f32(p);
     }
-    for (int l = 0; l < kMaxLevels && st == HPCG_B200_OK; ++l) {
-      float* v = nullptr;
-      if (l < p->nlev) {
-        const Level& L = p->lev[l];
-        const int64_t cnt = (int64_t)kSlots * L.pitch;
-        st = dev_alloc((void**)&v, sizeof(float) * cnt, &B->bytes);
-        if (st == HPCG_B200_OK) {
-          k_narrow<<<grid_for(c, cnt, kThreads, 8), kThreads, 0, c->stream>>>(v, L.val, cnt);
-          if (cudaGetLastError() != cudaSuccess) st = HPCG_B200_ERR_CUDA;
-        }
-      }
-      B->val32.push_back(v);
-    }
   }
   if (st == HPCG_B200_OK) {
-    std::vector<BGs> gs, gsb;
-    std::vector<BRes> res;
-    std::vector<BTile> tiles, btiles;
-    build_vcycle(B, 0, gs, res, tiles, gsb, btiles);
     std::vector<BVec> vec(count);
     std::vector<BTile> vt;
     std::vector<int> range(count + 1, 0);
@@ -1017,22 +1248,12 @@ int hpcg_b200_batch_create(int count, const int* nx, const int* ny, const int* n
     }
     range[count] = (int)vt.size();
     B->nvt = (int)vt.size();
-    st = alloc_copy(B, (void**)&B->gs_items, gs.data(), sizeof(BGs) * gs.size());
-    if (!st && !res.empty()) st = alloc_copy(B, (void**)&B->res_items, res.data(), sizeof(BRes) * res.size());
-    if (!st) st = alloc_copy(B, (void**)&B->tiles, tiles.data(), sizeof(BTile) * tiles.size());
-    if (!st) st = alloc_copy(B, (void**)&B->gs_bitems, gsb.data(), sizeof(BGs) * gsb.size());
-    if (!st) st = alloc_copy(B, (void**)&B->btiles, btiles.data(), sizeof(BTile) * btiles.size());
-    if (!st) st = alloc_copy(B, (void**)&B->vec, vec.data(), sizeof(BVec) * vec.size());
+    st = alloc_copy(B, (void**)&B->vec, vec.data(), sizeof(BVec) * vec.size());
     if (!st) st = alloc_copy(B, (void**)&B->vtiles, vt.data(), sizeof(BTile) * vt.size());
     if (!st) st = alloc_copy(B, (void**)&B->vrange, range.data(), sizeof(int) * range.size());
     if (!st) st = dev_alloc((void**)&B->partials, sizeof(double) * 2 * B->nvt, &B->bytes);
     if (!st) st = dev_alloc((void**)&B->sc, sizeof(BScal) * count, &B->bytes);
     if (!st) st = dev_alloc((void**)&B->ctl, sizeof(BCtl), &B->bytes);
-    if (!st) {
-      std::vector<DStep> ds;
-      for (const Step& x : B->steps) ds.push_back(DStep{x.kind, x.tile_off, x.ntiles});
-      st = alloc_copy(B, (void**)&B->dsteps, ds.data(), sizeof(DStep) * ds.size());
-    }
     if (!st) st = dev_alloc((void**)&B->bar, sizeof(BBar), &B->bytes);
     if (!st && cudaMemset(B->bar, 0, sizeof(BBar)) != cudaSuccess) st = HPCG_B200_ERR_CUDA;
     if (!st) {
@@ -1049,6 +1270,8 @@ int hpcg_b200_batch_create(int count, const int* nx, const int* ny, const int* n
     if (!st && cudaMallocHost(&B->sc_host, sizeof(BScal) * count) != cudaSuccess) st = HPCG_B200_ERR_NOMEM;
     if (!st && cudaMemset(B->sc, 0, sizeof(BScal) * count) != cudaSuccess) st = HPCG_B200_ERR_CUDA;
     if (!st) st = choose_form(B);
+    if (!st) st = B->bulk ? build_form1(B) : build_register_forms(B);
+    if (!st) st = stream_sync(c);
   }
   if (st != HPCG_B200_OK) {
     destroy(B);

@@ -81,9 +81,8 @@ __global__ void k_tail_values(const double* __restrict__ val, int64_t pitch, dou
 }
 
 template <typename T>
-bool launch(hpcg_b200_problem* p, int l, int nlev, const T* rhs, T* x, bool step) {
-  Context* c = p->ctx;
-  TailDesc<T> D;
+int describe(hpcg_b200_problem* p, int l, int nlev, TailDesc<T>* desc, size_t* smem) {
+  TailDesc<T>& D = *desc;
   std::memset(&D, 0, sizeof(D));
   D.nlev = nlev;
   int cluster = 1;
@@ -119,18 +118,23 @@ bool launch(hpcg_b200_problem* p, int l, int nlev, const T* rhs, T* x, bool step
   }
   D.elems = (int)((elems + 1) & ~1ll);  // the row table behind it: 8-byte aligned
   D.rows = (int)rows;
+  *smem = sizeof(T) * (size_t)D.elems + sizeof(TailRow) * (size_t)D.rows;
   int size = 1;
   while (size < cluster) size *= 2;
+  return size;
+}
+
+template <typename T>
+bool launch(hpcg_b200_problem* p, int l, int nlev, const T* rhs, T* x, bool step) {
+  Context* c = p->ctx;
+  TailDesc<T> D;
+  size_t smem = 0;
+  const int size = describe(p, l, nlev, &D, &smem);
   auto k = k_tail<T>;
-  const size_t smem = sizeof(T) * (size_t)D.elems + sizeof(TailRow) * (size_t)D.rows;
   static std::atomic<uint64_t> attr_set{0};
   const uint64_t bit = 1ull << c->device;
   if (!(attr_set.load(std::memory_order_acquire) & bit)) {
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-      set_error("k_tail attributes", cudaGetLastError());
-      return false;
-    }
+    if (tail_attributes((const void*)k, kMaxSmem) != HPCG_B200_OK) return false;
     attr_set.fetch_or(bit, std::memory_order_release);
   }
   cudaLaunchConfig_t cfg;
@@ -191,6 +195,18 @@ int tail_values(hpcg_b200_problem* p, int l) {
   }
   k_tail_values<<<grid_for(c, (int64_t)kSlots * L.pitch, 256, 8), 256, 0, c->stream>>>(L.val, L.pitch, L.valt);
   HB_CK(cudaGetLastError());
+  return HPCG_B200_OK;
+}
+
+int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<double>* D, size_t* smem) {
+  return describe(p, l, nlev, D, smem);
+}
+int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<float>* D, size_t* smem) {
+  return describe(p, l, nlev, D, smem);
+}
+int tail_attributes(const void* kernel, size_t smem) {
+  HB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  HB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return HPCG_B200_OK;
 }
 

@@ -65,6 +65,11 @@ __device__ __forceinline__ unsigned cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ unsigned cluster_blocks() {
+  unsigned n;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+  return n;
+}
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
@@ -401,5 +406,12 @@ __global__ void __launch_bounds__(kTailThreads, 1)
     k_tail(const __grid_constant__ TailDesc<T> D, const T* __restrict__ rhs, T* x, int step, unsigned* fault) {
   tail_run<T>(D, rhs, x, step != 0, fault);
 }
+
+// Host side (tail.cu). tail_desc: the description of problem p's levels l ..
+// l + nlev - 1, the shared memory of a block; returns the blocks of a cluster (a
+// power of two). tail_attributes: lets a kernel built on tail_run use it.
+int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<double>* D, size_t* smem);
+int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<float>* D, size_t* smem);
+int tail_attributes(const void* kernel, size_t smem);
 
 }  // namespace hb
