@@ -125,39 +125,57 @@ struct alignas(32) BGeoTile {
 
 using BatchShape = GsShape<float, kPackGeo>;
 
-// A full-slot phase: the single-problem FP32 phase's pipeline and shape.
+// Descriptions kept on chip by the kernels below; those of further problems are
+// read from memory. (Read from memory by every thread a full-slot phase of 0.5 M rows
+// took 22 us, with the list walked by the producer alone and this 20.)
+constexpr int kGeoCache = 24;
+
+// A full-slot phase: the single-problem FP32 phase's pipeline and shape. Items
+// item0 .. item0 + nitems - 1.
 __global__ void __launch_bounds__(BatchShape::threads, 1)
-    k_b_gs_geo(const BGeo* __restrict__ items, const BGeoTile* __restrict__ tiles, int ntiles,
+    k_b_gs_geo(const BGeo* __restrict__ items, int item0, int nitems, const BGeoTile* __restrict__ tiles, int ntiles,
                const BScal* __restrict__ sc, unsigned* fault) {
-  bulk_tiles_src<float, BatchShape, true>(
+  __shared__ BGeo cache[kGeoCache];
+  const int words = min(nitems, kGeoCache) * (int)(sizeof(BGeo) / sizeof(int));
+  for (int i = threadIdx.x; i < words; i += blockDim.x)
+    reinterpret_cast<int*>(cache)[i] = reinterpret_cast<const int*>(items + item0)[i];
+  bulk_tiles_driven<float, BatchShape>(
       ntiles,
       [&](int t) {
         const BGeoTile tl = tiles[t];
-        return TileSrc<float>{tl.start, tl.vals, nullptr, nullptr, 0};
+        TileSrc<float> ts{};
+        ts.q0 = (int64_t)(tl.item - item0) << 32 | (unsigned)tl.start;
+        ts.vals = tl.vals;
+        return ts;
       },
       [&](int t) { return !sc[tiles[t].prob].active; },
-      [&](int t, int64_t q0, const float* sv, const int*, int row, auto&& release) {
-        const BGeo& it = items[tiles[t].item];
-        const int q = (int)q0 + row;
+      [&](int64_t tag, const float* sv, int row, auto&& release) {
+        const int at = (int)(tag >> 32), q = (int)(unsigned)tag + row;
         float a[kSlots];
 #pragma unroll
-        for (int k = 0; k < kSlots; ++k) a[k] = sv[k * kBulkRows + row];
+        for (int k = 0; k < kSlots; ++k) a[k] = sv[k * kBulkRows];
         release();
-        if (q < it.r0 || q >= it.r1) return;
-        const GeoRow g(it.geo, q);
-        const float* x = it.x;
-        const int sink = it.sink;
-        float sum = it.rhs[q], xd = 0.0f;
+        auto work = [&](const BGeo& it) {
+          if (q < it.r0 || q >= it.r1) return;
+          const GeoRow g(it.geo, q);
+          const float* x = it.x;
+          const int sink = it.sink;
+          float sum = it.rhs[q], xd = 0.0f;
 #pragma unroll
-        for (int k = 0; k < kSlots; ++k) {
-          const float xv = __ldg(x + g.col(it.geo, k, sink));
-          sum -= a[k] * xv;
-          if (k == kDiagSlot) xd = xv;
-        }
-        sum += xd * a[kDiagSlot];
-        it.x[q] = sum / a[kDiagSlot];
+          for (int k = 0; k < kSlots; ++k) {
+            const float xv = __ldg(x + g.col(it.geo, k, sink));
+            sum -= a[k] * xv;
+            if (k == kDiagSlot) xd = xv;
+          }
+          sum += xd * a[kDiagSlot];
+          it.x[q] = sum / a[kDiagSlot];
+        };
+        if (at < kGeoCache)
+          work(cache[at]);
+        else
+          work(items[item0 + at]);
       },
-      fault, nullptr, nullptr);
+      fault);
 }
 
 // A first-sweep phase (k_gs_first_geo's arithmetic), 256 rows a tile.
@@ -226,38 +244,71 @@ __global__ void __launch_bounds__(kTailThreads, 2)
   tail_run<float>(D, D.lev[0].r, D.lev[0].x, false, fault);
 }
 
-// y = A x and partials of x'y per tile (b_spmv's arithmetic), columns from the grid.
-__global__ void __launch_bounds__(kThreads, 2)
-    k_b_spmv_geo(const BVec* __restrict__ v, const GeoGrid* __restrict__ grids, const BTile* __restrict__ tiles,
-                 int ntiles, const BScal* __restrict__ sc, double* __restrict__ partials) {
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile tl = tiles[t];
-    const BVec& it = v[tl.item];
-    double acc = 0.0;
-    const int q = tl.start + threadIdx.x;
-    if (sc[tl.item].active && q < it.n) {
-      double a[kSlots];
+// Ap = A p (b_spmv's arithmetic) on the single-problem SpMV's pipeline, columns
+// from the grid; one partial of p'Ap per warp: problem i's from 4 * tile0[i] on,
+// four to each of its 128-row tiles. (Sides are multiples of 16, so every
+// 256-row tile of the other kernels is two whole ones of these, and
+// k_b_finalize_warps sums the partials in those kernels' order: the FP32
+// V-cycle's input turns a last-bit difference of a dot into 1e-7 of a residual.)
+using BatchSpmv = SpmvShape<double, kPackGeo>;
+constexpr int kGridCache = 16;
+struct alignas(64) BMap {
+  CUtensorMap map;
+};
+__global__ void __launch_bounds__(BatchSpmv::threads, 1)
+    k_b_spmv_geo(const BVec* __restrict__ v, const GeoGrid* __restrict__ grids, int m, const BMap* __restrict__ maps,
+                 const BTile* __restrict__ tiles, int ntiles, const int* __restrict__ tile0,
+                 const BScal* __restrict__ sc, double* __restrict__ partials, unsigned* fault) {
+  __shared__ GeoGrid cache[kGridCache];
+  const int words = min(m, kGridCache) * (int)(sizeof(GeoGrid) / sizeof(int));
+  for (int i = threadIdx.x; i < words; i += blockDim.x)
+    reinterpret_cast<int*>(cache)[i] = reinterpret_cast<const int*>(grids)[i];
+  bulk_tiles_driven<double, BatchSpmv>(
+      ntiles,
+      [&](int t) {
+        const BTile tl = tiles[t];
+        TileSrc<double> ts{};
+        ts.q0 = (int64_t)tl.item << 32 | (unsigned)tl.start;
+        ts.map = &maps[tl.item].map;
+        return ts;
+      },
+      [&](int t) { return !sc[tiles[t].item].active; },
+      [&](int64_t tag, const double* sv, int row, auto&& release) {
+        const int p = (int)(tag >> 32), q0 = (int)(unsigned)tag, q = q0 + row;
+        double a[kSlots];
 #pragma unroll
-      for (int k = 0; k < kSlots; ++k) a[k] = __ldcs(it.val + k * it.pitch + q);
-      const GeoGrid& G = grids[tl.item];
-      int at = 0;
+        for (int k = 0; k < kSlots; ++k) a[k] = sv[k * kBulkRows];
+        release();
+        const int n = v[p].n;
+        const double* x = v[p].p;
+        double acc = 0.0;
+        auto work = [&](const GeoGrid& G) {
+          int at = 0;
 #pragma unroll
-      for (int s = 1; s < kColours; ++s) at += q >= G.block[s].start ? 1 : 0;
-      const GeoPhase& b = G.block[at];
-      const GeoRow g(b, q);
-      double sum = 0.0, xq = 0.0;
+          for (int s = 1; s < kColours; ++s) at += q >= G.block[s].start ? 1 : 0;
+          const GeoPhase& b = G.block[at];
+          const GeoRow g(b, q);
+          double sum = 0.0, xq = 0.0;
 #pragma unroll
-      for (int k = 0; k < kSlots; ++k) {
-        const double xv = __ldg(it.p + g.col(b, k, it.n));
-        sum += a[k] * xv;
-        if (k == kDiagSlot) xq = xv;
-      }
-      it.Ap[q] = sum;
-      acc = xq * sum;
-    }
-    const double s = block_sum(acc);
-    if (threadIdx.x == 0) partials[t] = s;
-  }
+          for (int k = 0; k < kSlots; ++k) {
+            const double xv = __ldg(x + g.col(b, k, n));
+            sum += a[k] * xv;
+            if (k == kDiagSlot) xq = xv;
+          }
+          v[p].Ap[q] = sum;
+          acc = xq * sum;
+        };
+        if (q < n) {
+          if (p < kGridCache)
+            work(cache[p]);
+          else
+            work(grids[p]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        if ((threadIdx.x & 31) == 0) partials[4 * (tile0[p] + q0 / kBulkRows) + row / 32] = acc;
+      },
+      fault);
 }
 
 // rc = (rf - A xf) at the injected rows (ComputeMG_ref.cpp:49-51, sorted pairs)
@@ -445,19 +496,94 @@ __global__ void __launch_bounds__(kThreads) k_b_update_xr(const BVec* __restrict
                                                           int ntiles, const BScal* __restrict__ sc,
                                                           double* __restrict__ partials) { b_update_xr(v, tiles, ntiles, sc, partials); }
 
+// ---- form 1's vector steps: the arithmetic of b_to64_dots and b_update_xr, with
+// the partials left per warp (summed by k_b_finalize_warps in the same order)
+// instead of two block barriers a tile, and r narrowed for the next V-cycle where
+// it is made.
+__global__ void __launch_bounds__(kThreads) k_b_to64_dots_w(const BVec* __restrict__ v,
+                                                            const BTile* __restrict__ tiles, int ntiles,
+                                                            const BScal* __restrict__ sc,
+                                                            double* __restrict__ partials) {
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const BTile tl = tiles[t];
+    if (!sc[tl.item].active) continue;  // its sums are not read
+    const BVec& it = v[tl.item];
+    const int q = tl.start + threadIdx.x;
+    double a1 = 0.0, a2 = 0.0;
+    if (q < it.n) {
+      const double z = (double)it.x32[q];
+      it.z[q] = z;
+      const double r = it.r[q];
+      a1 = r * z;
+      a2 = r * it.zprev[q];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a1 += __shfl_down_sync(0xffffffffu, a1, o);
+      a2 += __shfl_down_sync(0xffffffffu, a2, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      const int64_t w = 8 * (int64_t)t + (threadIdx.x >> 5);
+      partials[w] = a1;
+      partials[8 * (int64_t)ntiles + w] = a2;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kThreads) k_b_update_xr_w(const BVec* __restrict__ v,
+                                                            const BTile* __restrict__ tiles, int ntiles,
+                                                            const BScal* __restrict__ sc,
+                                                            double* __restrict__ partials) {
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const BTile tl = tiles[t];
+    if (!sc[tl.item].active) continue;  // its norm stays
+    const BVec& it = v[tl.item];
+    const int q = tl.start + threadIdx.x;
+    double acc = 0.0;
+    if (q < it.n) {
+      const double alpha = sc[tl.item].alpha;
+      it.x[q] = it.x[q] + alpha * it.p[q];
+      const double r = it.r[q] + -alpha * it.Ap[q];
+      it.r[q] = r;
+      it.r32[q] = (float)r;
+      acc = r * r;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) partials[8 * (int64_t)t + (threadIdx.x >> 5)] = acc;
+  }
+}
+
 enum BFin : int { kBNorm0 = 0, kBRtz = 1, kBPap = 2, kBNormr = 3 };
 
+// The sum of a 256-row tile from its eight warps' sums, in block_sum's order.
+__device__ __forceinline__ double tile_of_warps(const double* __restrict__ w) {
+  return ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+}
+
 // Problem p's fixed-order sum over its tiles, then its scalar step; block b
-// takes problems b, b + gridDim.x, ...
+// takes problems b, b + gridDim.x, ... WARPS: the partials are the tiles' warps'.
+template <bool WARPS = false>
 __device__ __forceinline__ void b_finalize(BScal* sc, const double* __restrict__ partials, int ntiles,
                                            const int* __restrict__ range, int op, const BCtl* __restrict__ ctl,
                                            int m) {
   for (int p = blockIdx.x; p < m; p += gridDim.x) {
     const int t0 = range[p], t1 = range[p + 1];
+    if (WARPS && !sc[p].active) continue;  // no sums were left for it, and its scalars stay
     double a1 = 0.0, a2 = 0.0;
-    for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
-      a1 += partials[t];
-      if (op == kBRtz) a2 += partials[ntiles + t];
+    if (WARPS) {
+#pragma unroll 4
+      for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) a1 += tile_of_warps(partials + 8 * (int64_t)t);
+      if (op == kBRtz) {
+#pragma unroll 4
+        for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x)
+          a2 += tile_of_warps(partials + 8 * ((int64_t)ntiles + t));
+      }
+    } else {
+      for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
+        a1 += partials[t];
+        if (op == kBRtz) a2 += partials[ntiles + t];
+      }
     }
     const double s1 = block_sum(a1);
     const double s2 = op == kBRtz ? block_sum(a2) : 0.0;
@@ -499,6 +625,11 @@ __device__ __forceinline__ void b_finalize(BScal* sc, const double* __restrict__
 }
 
 // One block per problem.
+__global__ void __launch_bounds__(kThreads) k_b_finalize_warps(BScal* sc, const double* __restrict__ partials,
+                                                               int ntiles, const int* __restrict__ range, int op,
+                                                               const BCtl* __restrict__ ctl, int m) {
+  b_finalize<true>(sc, partials, ntiles, range, op, ctl, m);
+}
 __global__ void __launch_bounds__(kThreads) k_b_finalize(BScal* sc, const double* __restrict__ partials,
                                                          int ntiles, const int* __restrict__ range, int op,
                                                          const BCtl* __restrict__ ctl, int m) {
@@ -677,6 +808,8 @@ struct GeoStep {
   int s;         // kFirst: sweep position
   int tile_off;  // first tile
   int ntiles;
+  int item_off;  // kFull: first item, items
+  int nitems;
 };
 
 }  // namespace
@@ -699,7 +832,13 @@ struct hpcg_b200_batch {
   hb::BGeoTile* geo_tiles;
   hb::BRes* prolong_items;
   hb::BTile* prolong_tiles;
-  hb::GeoGrid* grids;            // [m] level 0
+  hb::GeoGrid* grids;            // [m] level 0, and its tensor map
+  hb::BMap* maps;
+  hb::BTile* mv_tiles;           // 128-row tiles of every problem's level 0
+  int mv_ntiles;
+  int* mv_tile0;                 // [m + 1] first of each problem
+  double* mv_partials;
+  std::vector<int> tail_at;      // first level in the one-launch part
   hb::TailDesc<float>* descs;    // [m] the small levels (nlev 0: none)
   std::vector<hb::GeoStep> geo_steps;
   int tail_cluster;              // blocks of a cluster
@@ -827,15 +966,15 @@ void build_geo(hpcg_b200_batch* B, int l, GeoLists& W) {
   const int m = B->m;
   std::vector<int> in;
   for (int p = 0; p < m; ++p)
-    if (l < kMaxLevels && tail_first(B->probs[p], true) > l) in.push_back(p);
+    if (l < kMaxLevels && B->tail_at[p] > l) in.push_back(p);
   if (in.empty() || l >= kMaxLevels) {  // the others' levels are done above: now the small ones of all
     bool any = false;
-    for (int p = 0; p < m; ++p) any = any || tail_first(B->probs[p], true) < B->probs[p]->nlev;
-    if (any) B->geo_steps.push_back(GeoStep{GeoStep::kTail, 0, 0, 0});
+    for (int p = 0; p < m; ++p) any = any || B->tail_at[p] < B->probs[p]->nlev;
+    if (any) B->geo_steps.push_back(GeoStep{GeoStep::kTail, 0, 0, 0, 0, 0});
     return;
   }
   auto step = [&](GeoStep::Kind kind, int s, int rows) {
-    GeoStep st{kind, s, (int)W.tiles.size(), 0};
+    GeoStep st{kind, s, (int)W.tiles.size(), 0, (int)W.items.size(), (int)in.size()};
     for (int p : in) {
       const Level& L = B->probs[p]->lev[l];
       const int item = (int)W.items.size();
@@ -868,7 +1007,7 @@ void build_geo(hpcg_b200_batch* B, int l, GeoLists& W) {
   if (l + 1 < kMaxLevels) {
     step(GeoStep::kRestrict, kColours - 1, kTile);
     build_geo(B, l + 1, W);
-    GeoStep st{GeoStep::kProlong, 0, (int)W.rtiles.size(), 0};
+    GeoStep st{GeoStep::kProlong, 0, (int)W.rtiles.size(), 0, 0, 0};
     for (int p : in) {
       const Level& L = B->probs[p]->lev[l];
       const Level& C = B->probs[p]->lev[l + 1];
@@ -938,8 +1077,8 @@ int launch_geo_step(hpcg_b200_batch* B, const GeoStep& st) {
       // (a first-sweep phase, a prolongation) of every V-cycle
       attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attr[0].val.programmaticStreamSerializationAllowed = 1;
-      HB_CK(cudaLaunchKernelEx(&cfg, k_b_gs_geo, (const BGeo*)B->geo_items, tiles, st.ntiles, (const BScal*)B->sc,
-                               c->fault));
+      HB_CK(cudaLaunchKernelEx(&cfg, k_b_gs_geo, (const BGeo*)B->geo_items, st.item_off, st.nitems, tiles, st.ntiles,
+                               (const BScal*)B->sc, c->fault));
       return HPCG_B200_OK;
     }
     case GeoStep::kFirst:
@@ -982,24 +1121,45 @@ int finalize_b(hpcg_b200_batch* B, int op) {
   return HPCG_B200_OK;
 }
 
-// one flexible-CG iteration of every active problem
+int finalize_w(hpcg_b200_batch* B, int op) {
+  k_b_finalize_warps<<<B->m, kThreads, 0, B->ctx->stream>>>(B->sc, B->mv_partials, B->nvt, B->vrange, op, B->ctl,
+                                                            B->m);
+  HB_CK(cudaGetLastError());
+  return HPCG_B200_OK;
+}
+
+// one flexible-CG iteration of every active problem, form 1 (r32 holds r)
+int iteration_geo(hpcg_b200_batch* B) {
+  Context* c = B->ctx;
+  const int gv = grid_tiles(c, B->nvt);
+  for (const GeoStep& s : B->geo_steps) HB_TRY(launch_geo_step(B, s));
+  k_b_to64_dots_w<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->mv_partials);
+  HB_CK(cudaGetLastError());
+  HB_TRY(finalize_w(B, kBRtz));
+  k_b_update_p<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->ctl);
+  static std::atomic<uint64_t> attr_set{0};  // devices on which the shared-memory size is enabled
+  bulk_attr(k_b_spmv_geo, BatchSpmv::smem, c->device, &attr_set);
+  k_b_spmv_geo<<<std::min(B->mv_ntiles, c->sms), BatchSpmv::threads, BatchSpmv::smem, c->stream>>>(
+      B->vec, B->grids, B->m, B->maps, B->mv_tiles, B->mv_ntiles, B->mv_tile0, B->sc, B->mv_partials, c->fault);
+  HB_CK(cudaGetLastError());
+  HB_TRY(finalize_w(B, kBPap));
+  k_b_update_xr_w<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->mv_partials);
+  HB_CK(cudaGetLastError());
+  return finalize_w(B, kBNormr);
+}
+
+// ... and form 0
 int iteration(hpcg_b200_batch* B) {
   Context* c = B->ctx;
   const int gv = grid_tiles(c, B->nvt);
   k_b_to32<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc);
   HB_CK(cudaGetLastError());
-  if (B->bulk)
-    for (const GeoStep& s : B->geo_steps) HB_TRY(launch_geo_step(B, s));
-  else
-    for (const Step& s : B->steps) HB_TRY(launch_step(B, s));
+  for (const Step& s : B->steps) HB_TRY(launch_step(B, s));
   k_b_to64_dots<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->partials);
   HB_CK(cudaGetLastError());
   HB_TRY(finalize_b(B, kBRtz));
   k_b_update_p<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->ctl);
-  if (B->bulk)
-    k_b_spmv_geo<<<gv, kThreads, 0, c->stream>>>(B->vec, B->grids, B->vtiles, B->nvt, B->sc, B->partials);
-  else
-    k_b_spmv<true><<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, 1, B->sc, B->partials);
+  k_b_spmv<true><<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, 1, B->sc, B->partials);
   HB_CK(cudaGetLastError());
   HB_TRY(finalize_b(B, kBPap));
   k_b_update_xr<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc, B->partials);
@@ -1088,7 +1248,7 @@ int build_graph(hpcg_b200_batch* B) {
     if (e != cudaSuccess) set_error("batch graph", e);
     return st != HPCG_B200_OK ? st : status_of(e);
   }
-  st = B->persist ? launch_iteration(B, false) : iteration(B);
+  st = B->persist ? launch_iteration(B, false) : B->bulk ? iteration_geo(B) : iteration(B);
   if (st == HPCG_B200_OK) {
     k_b_condition<<<1, 32, 0, c->stream>>>(B->ctl, B->sc, B->m, h, 1, B->bar, c->fault);
     if (cudaGetLastError() != cudaSuccess) st = HPCG_B200_ERR_CUDA;
@@ -1111,21 +1271,34 @@ int build_graph(hpcg_b200_batch* B) {
 // stored ones), else 0, one launch per step on the register kernels.
 // HPCG_B200_BATCH_PERSIST=1: 2, the whole iteration as one cooperative launch;
 // HPCG_B200_BATCH_BULK=0 (or PERSIST=0 without BULK=1): 0. Sixteen problems of
-// sides 32 to 128: form 1 takes BATCH_FORM1 ms to 1e-9, form 0 105.
+// sides 32 to 128: form 1 takes 54 ms to 1e-9, form 0 105.
 int choose_form(hpcg_b200_batch* B) {
   const char* fp = std::getenv("HPCG_B200_BATCH_PERSIST");
   const char* fb = std::getenv("HPCG_B200_BATCH_BULK");
   bool geo = true;
   for (hpcg_b200_problem* p : B->probs)
-    for (int l = 0; l < p->nlev; ++l) geo = geo && p->lev[l].geo_cols && p->lev[l].tf_run >= (l + 1 < p->nlev ? 0 : -1);
+    for (int l = 0; l < p->nlev; ++l) geo = geo && p->lev[l].geo_cols && (l + 1 == p->nlev || p->lev[l].tf_run >= 0);
+  for (hpcg_b200_problem* p : B->probs) geo = geo && bulk_maps(p->lev[0]) != nullptr;
   const bool want = fb && *fb ? std::atoi(fb) != 0 : !(fp && *fp);
   B->persist = fp && *fp && std::atoi(fp) != 0 && B->persist_grid > 0;
   B->bulk = !B->persist && geo && want;
   return HPCG_B200_OK;
 }
 
+constexpr int kBatchTailRows = 1280;
+
 // Form 1's work lists.
 int build_form1(hpcg_b200_batch* B) {
+  // One cut for all problems, the first level at which every problem fits: a
+  // level that some problem needs launches for costs the others' rows little
+  // there, and the one-launch part as long as its longest cluster. There the
+  // problems run side by side, so up to five chunks of rows a phase (2.2 us)
+  // still beat a launch for every phase. With more clusters than the GPU holds
+  // at one block to an SM, two blocks share one.
+  int cut = 0;
+  for (hpcg_b200_problem* p : B->probs)
+    cut = std::max(cut, tail_first_within(p, true, kBatchTailRows, B->m > 8 ? 110 * 1024 : 200 * 1024));
+  B->tail_at.assign(B->m, cut);
   GeoLists W;
   build_geo(B, 0, W);
   std::vector<TailDesc<float>> descs(B->m);
@@ -1136,7 +1309,7 @@ int build_form1(hpcg_b200_batch* B) {
     hpcg_b200_problem* P = B->probs[p];
     grids.push_back(*P->lev[0].geo_cols);
     std::memset(&descs[p], 0, sizeof(descs[p]));
-    const int l = tail_first(P, true);
+    const int l = B->tail_at[p];
     if (l < P->nlev) {
       size_t smem = 0;
       B->tail_cluster = std::max(B->tail_cluster, tail_desc(P, l, P->nlev - l, &descs[p], &smem));
@@ -1149,6 +1322,20 @@ int build_form1(hpcg_b200_batch* B) {
   HB_TRY(alloc_copy(B, (void**)&B->prolong_items, W.res.data(), sizeof(BRes) * W.res.size()));
   HB_TRY(alloc_copy(B, (void**)&B->prolong_tiles, W.rtiles.data(), sizeof(BTile) * W.rtiles.size()));
   HB_TRY(alloc_copy(B, (void**)&B->grids, grids.data(), sizeof(GeoGrid) * grids.size()));
+  std::vector<BMap> maps(B->m);
+  std::vector<BTile> mv;
+  std::vector<int> tile0(B->m + 1, 0);
+  for (int p = 0; p < B->m; ++p) {
+    const Level& L = B->probs[p]->lev[0];
+    std::memcpy(&maps[p].map, &bulk_maps(L)->val, sizeof(CUtensorMap));
+    for (int q = 0; q < L.n; q += kBulkRows) mv.push_back(BTile{p, q});
+    tile0[p + 1] = (int)mv.size();
+  }
+  B->mv_ntiles = (int)mv.size();
+  HB_TRY(alloc_copy(B, (void**)&B->maps, maps.data(), sizeof(BMap) * maps.size()));
+  HB_TRY(alloc_copy(B, (void**)&B->mv_tiles, mv.data(), sizeof(BTile) * mv.size()));
+  HB_TRY(alloc_copy(B, (void**)&B->mv_tile0, tile0.data(), sizeof(int) * tile0.size()));
+  HB_TRY(dev_alloc((void**)&B->mv_partials, sizeof(double) * 16 * B->nvt, &B->bytes));  // two sums, 8 warps a tile
   return alloc_copy(B, (void**)&B->descs, descs.data(), sizeof(TailDesc<float>) * descs.size());
 }
 
@@ -1186,7 +1373,7 @@ void destroy(hpcg_b200_batch* B) {
   if (B->ctx) cudaStreamSynchronize(B->ctx->stream);
   if (B->graph) cudaGraphExecDestroy(B->graph);
   void* v[] = {B->gs_items, B->res_items, B->tiles, B->geo_items, B->geo_tiles, B->prolong_items, B->prolong_tiles,
-               B->grids, B->descs, B->vec, B->vtiles, B->vrange, B->partials, B->sc, B->ctl, B->dsteps, B->bar};
+               B->grids, B->maps, B->mv_tiles, B->mv_tile0, B->mv_partials, B->descs, B->vec, B->vtiles, B->vrange, B->partials, B->sc, B->ctl, B->dsteps, B->bar};
   for (void* q : v) cudaFree(q);
   for (float* q : B->val32) cudaFree(q);
   if (B->sc_host) cudaFreeHost(B->sc_host);
@@ -1220,6 +1407,8 @@ int hpcg_b200_batch_create(int count, const int* nx, const int* ny, const int* n
   B->m = count;
   B->gs_items = nullptr; B->res_items = nullptr; B->tiles = nullptr; B->vec = nullptr; B->vtiles = nullptr;
   B->geo_items = nullptr; B->geo_tiles = nullptr; B->prolong_items = nullptr; B->prolong_tiles = nullptr;
+  B->maps = nullptr; B->mv_tiles = nullptr; B->mv_tile0 = nullptr; B->mv_partials = nullptr;
+  B->mv_ntiles = 0;
   B->grids = nullptr; B->descs = nullptr; B->bulk = false; B->tail_cluster = 1; B->tail_smem = 0;
   B->persist = false; B->persist_grid = 0; B->dsteps = nullptr; B->bar = nullptr;
   B->vrange = nullptr; B->partials = nullptr; B->sc = nullptr; B->sc_host = nullptr; B->ctl = nullptr;
@@ -1307,6 +1496,10 @@ int hpcg_b200_batch_cg_mixed(hpcg_b200_batch* B, const double* const* b, double*
   k_b_resid<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->partials);
   HB_CK(cudaGetLastError());
   HB_TRY(finalize_b(B, kBNorm0));
+  if (B->bulk) {
+    k_b_to32<<<gv, kThreads, 0, c->stream>>>(B->vec, B->vtiles, B->nvt, B->sc);
+    HB_CK(cudaGetLastError());
+  }
   if (!B->graph) {
     int gs = build_graph(B);
     if (gs != HPCG_B200_OK && B->persist) {  // a cooperative launch refused inside a capture

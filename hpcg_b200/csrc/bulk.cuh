@@ -358,6 +358,7 @@ struct TileSrc {
   const int* cols;
   const unsigned char* rec;
   int rec_bytes;
+  const CUtensorMap* map = nullptr;  // FP64 tiles of bulk_tiles_driven: the matrix the tile is of
 };
 
 // The producer/consumer pipeline of the bulk-copy kernels, run by the whole
@@ -492,6 +493,102 @@ __device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, R
         }
       }
       ++i;
+    }
+  }
+}
+
+// The same pipeline for work lists whose tiles come from several matrices and
+// may be skipped: the producer alone walks the list and tells each group what
+// it got, a tag (TileSrc::q0: the tile's first row in the low 32 bits, anything
+// not negative above) and at the end a negative one, so the consumers read
+// neither the list nor what decides the skipping. Columns from the grid (values
+// only), early release: row(tag, sv, t, release), t the row in the tile.
+template <typename T, typename Shape, typename Src, typename Skip, typename RowFn>
+__device__ __forceinline__ void bulk_tiles_driven(int ntiles, Src src, Skip skip, RowFn row, unsigned* fault) {
+  constexpr int G = Shape::groups;
+  constexpr int RING = Shape::ring;
+  constexpr int S = Shape::stages;
+  constexpr int SB = Shape::stage_bytes;
+  static_assert(Shape::geo && Shape::lanes == 1, "values only, one thread per row");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned char* smem = smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * SB);
+  uint64_t* empty = full + S;
+  int64_t* first = reinterpret_cast<int64_t*>(empty + S);  // the tag of the tile in each stage
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], Shape::group_threads);
+    }
+    mbar_init_fence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) griddep_launch_dependents();
+  const int warp = threadIdx.x >> 5;
+  if (warp == 0) {
+    if (threadIdx.x == 0) {
+      const uint64_t policy = evict_first_policy();
+      int last[S];  // last fill copied into each stage (-1: none)
+#pragma unroll
+      for (int s = 0; s < S; ++s) last[s] = -1;
+      int i = 0, ends = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; ok && ends < G; tile += gridDim.x) {
+        const bool end = tile >= ntiles;
+        if (!end && skip(tile)) continue;
+        const int kg = i / G;
+        const int s = (i % G) * RING + kg % RING, use = kg / RING;
+        TileSrc<T> ts{};
+        if (!end) ts = src(tile);
+        if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1)) {
+          record_fault(fault, 1);
+          ok = false;
+          break;
+        }
+        if (end) {
+          first[s] = -1;
+          mbar_arrive(&full[s]);
+          ++ends;
+          // (the wait above, or no fill at all: nothing is landing in this stage,
+          // and its barrier is past the fill's phase)
+#pragma unroll
+          for (int u = 0; u < S; ++u)
+            if (u == s) last[u] = -1;
+        } else {
+          first[s] = ts.q0;
+          mbar_expect_tx(&full[s], Shape::value_bytes);
+          T* sv = reinterpret_cast<T*>(smem + s * SB);
+          if constexpr (bulk_whole_tile<T>())
+            bulk_g2s(sv, ts.vals, Shape::value_bytes, &full[s], policy);
+          else
+            tma_load_2d(sv, ts.map, (int)(unsigned)ts.q0, 0, &full[s], policy);
+#pragma unroll
+          for (int u = 0; u < S; ++u)
+            if (u == s) last[u] = use;
+        }
+        ++i;
+      }
+      // no copy may still be landing when the block exits
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+        if (last[s] >= 0 && !mbar_wait(&full[s], last[s] & 1)) record_fault(fault, 2);
+    }
+    __syncwarp();
+  } else {
+    griddep_wait();
+    const int g = (warp - 1) / (Shape::group_threads / 32);
+    const int t = (threadIdx.x - 32) % Shape::group_threads;
+    for (int kg = 0;; ++kg) {
+      const int s = g * RING + kg % RING, use = kg / RING;
+      if (!mbar_wait(&full[s], use & 1)) {
+        record_fault(fault, 3);
+        break;
+      }
+      const int64_t tag = first[s];
+      if (tag < 0) break;
+      const int h = t / Shape::block_threads;
+      row(tag, reinterpret_cast<const T*>(smem + s * SB + h * Shape::block_value_bytes) + (t - h * Shape::block_threads),
+          t, [&] { mbar_arrive(&empty[s]); });
     }
   }
 }

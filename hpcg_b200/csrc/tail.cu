@@ -54,10 +54,20 @@ int64_t bytes_of(const Level& L, int act, bool f32) {
   return elems_of(L, act) * (f32 ? 4 : 8) + rows_of(L, act) * (int64_t)sizeof(TailRow);
 }
 
-bool level_fits(const Level& L, bool f32) {
-  if (!L.geo || L.next || L.n <= 0) return false;
-  const int act = blocks_of(L);
-  return most_rows(L, act) <= max_rows(f32) && bytes_of(L, act, f32) <= kMaxSmem;
+// the first level from which all levels fit a block's share of max_rows rows a
+// phase and max_bytes of shared memory
+int first_within(const hpcg_b200_problem* p, bool f32, int64_t rows, int64_t max_bytes) {
+  int64_t bytes = 256;  // rounding of the table's place
+  int f = p->nlev;
+  for (int l = p->nlev - 1; l >= 0; --l) {
+    const Level& L = p->lev[l];
+    if (!L.geo || L.next || L.n <= 0 || (l + 1 < p->nlev && !L.geo_f2c)) break;
+    const int act = blocks_of(L);
+    bytes += bytes_of(L, act, f32);
+    if (most_rows(L, act) > rows || bytes > max_bytes) break;
+    f = l;
+  }
+  return f;
 }
 
 // On unless the environment pins kernel configurations or asks for wavefront
@@ -167,20 +177,16 @@ int tail_first(hpcg_b200_problem* p, bool f32) {
   if (first >= 0) return first;
   first = p->nlev;
   if (!wanted()) return first;
-  int64_t bytes = 256;  // rounding of the table's place
-  int f = p->nlev;
-  for (int l = p->nlev - 1; l >= 0; --l) {
-    const Level& L = p->lev[l];
-    if (!level_fits(L, f32) || (l + 1 < p->nlev && !L.geo_f2c)) break;
-    bytes += bytes_of(L, blocks_of(L), f32);
-    if (bytes > kMaxSmem) break;
-    f = l;
-  }
+  const int f = first_within(p, f32, max_rows(f32), kMaxSmem);
   if (!f32)
     for (int l = f; l < p->nlev; ++l)
       if (!p->lev[l].valt && tail_values(p, l) != HPCG_B200_OK) return first;  // no memory: the phases run
   first = f;
   return first;
+}
+
+int tail_first_within(const hpcg_b200_problem* p, bool f32, int64_t rows, int64_t bytes) {
+  return wanted() ? first_within(p, f32, rows, std::min<int64_t>(bytes, kMaxSmem)) : p->nlev;
 }
 
 // The FP64 values of a small level in the layout tail.cuh reads, built (or,

@@ -154,10 +154,8 @@ struct alignas(16) TailPhase {
   uint32_t mask;  // first_mask
 };
 // A row's place: its element, marked if it lies in the first / last plane of
-// the slab with a block beyond, and the offset of its values.
-struct TailRow {
-  unsigned e, v;
-};
+// the slab with a block beyond.
+using TailRow = unsigned;
 constexpr unsigned kTailLow = 1u << 30, kTailHigh = 1u << 31;
 
 // A block's share of one level.
@@ -198,9 +196,8 @@ struct TailSlab {
   __device__ TailRow row(const TailPhase& P, int i) const {
     const int zz = i / P.per, rem = i - zz * P.per, yy = rem / P.hx, xx = rem - yy * P.hx;
     const int px = P.colour & 1, py = (P.colour >> 1) & 1, lz = 2 * zz + ((P.colour >> 2) & 1) + 1;
-    return {(unsigned)(lz * sh.sz + (2 * yy + py + 1) * sh.sy + px * sh.hx + xx + 1) |
-                (lz == 1 && rank > 0 ? kTailLow : 0u) | (lz == planes && rank + 1 < L.act ? kTailHigh : 0u),
-            (unsigned)mat_index<T, kTailBlock>(0, P.q0 + i, 0)};
+    return (unsigned)(lz * sh.sz + (2 * yy + py + 1) * sh.sy + px * sh.hx + xx + 1) |
+           (lz == 1 && rank > 0 ? kTailLow : 0u) | (lz == planes && rank + 1 < L.act ? kTailHigh : 0u);
   }
   // the row of the next level injected from the i-th row of the all-even points
   __device__ int coarse(const TailDesc<T>& D, const TailLevel<T>& C, const TailPhase& P, int i) const {
@@ -260,8 +257,8 @@ __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem,
   // sweep position of phase j: 0 .. 7, 6 .. 0, and the injected rows (position 7)
   auto pos_of = [](int j) { return j < 8 ? j : j < 15 ? 14 - j : 7; };
   // a row's 27 values
-  auto fetch = [&](T(&v)[kSlots + 1], unsigned at, const TailPhase& P, int j) {
-    const T* p = L.val + at;
+  auto fetch = [&](T(&v)[kSlots + 1], int q, const TailPhase& P, int j) {
+    const T* p = L.val + ((unsigned)q / kTailBlock * (kSlots * kTailBlock) + (unsigned)q % kTailBlock);
     if (ZERO && j < 8) {
       const uint32_t m = P.mask | 1u << kDiagSlot;
 #pragma unroll
@@ -275,13 +272,13 @@ __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem,
   int j = 0, i = tid;                // phase, this thread's row in it
   TailPhase P = tab[0];
   TailRow R = table[P.t0 + (i < P.cnt ? i : 0)];
-  fetch(va, R.v, P, 0);
+  fetch(va, P.q0 + (i < P.cnt ? i : 0), P, 0);
   cluster_sync_all();  // what the sweep reads (rhs, the next level's x) is written
   if (prolong) {
     const TailLevel<T>& C = D.lev[l + 1];
     const TailPhase PI = tab[7];
     for (int u = tid; u < PI.cnt; u += kTailThreads) {
-      const unsigned t = table[PI.t0 + u].e;
+      const unsigned t = table[PI.t0 + u];
       put(t, S.xs[t & ~(kTailLow | kTailHigh)] + __ldcg(C.x + S.coarse(D, C, PI, u)));
     }
     wait.end(rank, L.act, PI.sent);
@@ -301,14 +298,14 @@ __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem,
     if (more && ni - lane < NP.cnt) {
       const int nc = ni < NP.cnt ? ni : 0;
       NR = table[NP.t0 + nc];
-      fetch(next, NR.v, NP, nj);
+      fetch(next, NP.q0 + nc, NP, nj);
       next[kSlots] = __ldcg(rhs + NP.q0 + nc);
     }
     const bool res = j == 15;  // the residual at the injected rows
     if (i < P.cnt) {
       // the gathers' two bases: the row's own x parity, and the other one (the
       // neighbour at x - 1; the one at x + 1 is the next element)
-      const T* xp = S.xs + (R.e & ~(kTailLow | kTailHigh));
+      const T* xp = S.xs + (R & ~(kTailLow | kTailHigh));
       const T* xo = xp + (P.colour & 1 ? -S.sh.hx : S.sh.hx - 1);
       T xv[kSlots];
 #pragma unroll
@@ -328,7 +325,7 @@ __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem,
         const T d = a[kDiagSlot];
         if (!(ZERO && j < 8)) sum += xv[kDiagSlot] * d;
         const T out = sum / d;
-        put(R.e, out);
+        put(R, out);
         if (keep && j >= 7) xg[P.q0 + i] = out;
       }
     }
@@ -413,5 +410,8 @@ __global__ void __launch_bounds__(kTailThreads, 1)
 int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<double>* D, size_t* smem);
 int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<float>* D, size_t* smem);
 int tail_attributes(const void* kernel, size_t smem);
+// tail_first for other bounds than the single problem's: rows of a block in one
+// phase, bytes of its shared memory
+int tail_first_within(const hpcg_b200_problem* p, bool f32, int64_t rows, int64_t bytes);
 
 }  // namespace hb
