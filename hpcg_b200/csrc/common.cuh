@@ -347,6 +347,8 @@ enum ProfKind : int {
   kProfKinds = 7,
 };
 
+constexpr int kLoneSlots = 64, kLoneBytes = kLoneSlots * 16;
+
 struct Context {
   int device = -1;
   int sms = 0;
@@ -368,6 +370,11 @@ struct Context {
   double prof_ms[kProfKinds] = {};
   long prof_launches[kProfKinds] = {};
   int64_t prof_rows[kProfKinds] = {};                 // rows processed by the timed launches
+  // the lone reductions' arrival counter (device) and results (pinned, mapped),
+  // taken in turn by the calls
+  unsigned* lone_count = nullptr;
+  void* lone = nullptr;
+  std::atomic<unsigned long long> lone_call{0};
   // fault word of the kernels with bounded waits (pinned, mapped): nonzero once a
   // wait gave up; read and cleared by stream_sync
   unsigned* fault = nullptr;

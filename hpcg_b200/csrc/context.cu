@@ -96,6 +96,10 @@ Context* context_for(int device) {
   if (e == cudaSuccess) e = cudaMallocHost(&c->scal_host, sizeof(Scalars));
   if (e == cudaSuccess) e = cudaHostAlloc(&c->fault, sizeof(unsigned), cudaHostAllocMapped);
   if (e == cudaSuccess) *c->fault = 0;
+  if (e == cudaSuccess) e = cudaMalloc(&c->lone_count, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset(c->lone_count, 0, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaHostAlloc(&c->lone, kLoneBytes, cudaHostAllocMapped);
+  if (e == cudaSuccess) std::memset(c->lone, 0, kLoneBytes);
   if (e != cudaSuccess) {
     set_error("context set-up", e);
     if (c->stream) cudaStreamDestroy(c->stream);

@@ -799,6 +799,88 @@ __global__ void __launch_bounds__(kThreads) k_prolong(const int* __restrict__ tf
 
 // ---- vectors ----------------------------------------------------------------
 
+// Natural order <-> colour order by the grid: 16 bytes a row. (Through an index
+// array it is 20, and reading natural order in colour order uses half of each
+// sector: 128^3 9.8 us against 7.0.) Threads walk natural order; a warp's
+// neighbours lie in two colours, two runs.
+struct NatGrid {
+  int start[kColours];  // first row by parity colour
+  int hx[2], hy[2];     // half-sides by parity
+  int nx, ny, n;
+  FastDiv dx, dy;       // by nx, ny
+};
+inline NatGrid nat_grid(const ColourGrid& g, int n) {
+  NatGrid N;
+  for (int c = 0; c < kColours; ++c) N.start[c] = g.start[g.pos[c]];
+  for (int b = 0; b < 2; ++b) {
+    N.hx[b] = ColourGrid::half(g.nx, b);
+    N.hy[b] = ColourGrid::half(g.ny, b);
+  }
+  N.nx = g.nx;
+  N.ny = g.ny;
+  N.n = n;
+  N.dx.init((unsigned)g.nx);
+  N.dy.init((unsigned)g.ny);
+  return N;
+}
+__device__ __forceinline__ int nat_to_colour(const NatGrid& g, int i) {
+  const int t = (int)g.dx.div((unsigned)i), ix = i - t * g.nx;
+  const int iz = (int)g.dy.div((unsigned)t), iy = t - iz * g.ny;
+  const int px = ix & 1, py = iy & 1;
+  return g.start[px | py << 1 | (iz & 1) << 2] + ((iz >> 1) * g.hy[py] + (iy >> 1)) * g.hx[px] + (ix >> 1);
+}
+template <bool TO_COLOUR>
+__global__ void __launch_bounds__(kThreads) k_permute(double* __restrict__ dst, const double* __restrict__ src,
+                                                      const __grid_constant__ NatGrid g) {
+  constexpr int U = 4;  // rows in flight of a thread
+  const int stride = gridDim.x * kThreads;
+  for (int i0 = blockIdx.x * kThreads + threadIdx.x; i0 < g.n; i0 += U * stride) {
+    int q[U];
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * stride;
+      if (i < g.n) {
+        q[u] = nat_to_colour(g, i);
+        v[u] = TO_COLOUR ? src[i] : src[q[u]];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * stride;
+      if (i < g.n) dst[TO_COLOUR ? q[u] : i] = v[u];
+    }
+  }
+}
+
+// y = A x on natural-order vectors, columns and order from the grid: a call on a
+// grid is one launch instead of three (16^3 19.0 -> 14.4 us). Thread q has
+// colour-order row q, so the matrix streams; the vectors are strided by two.
+__global__ void __launch_bounds__(kThreads) k_spmv_nat(const double* __restrict__ val, int64_t pitch,
+                                                       const int* __restrict__ new2old,
+                                                       const double* __restrict__ x, double* __restrict__ y, int nx,
+                                                       int ny, int nz, FastDiv dx, FastDiv dy, int n) {
+  const int q = blockIdx.x * kThreads + threadIdx.x;
+  if (q >= n) return;
+  double a[kSlots];
+#pragma unroll
+  for (int k = 0; k < kSlots; ++k) a[k] = __ldcs(val + (int64_t)k * pitch + q);
+  const int i = new2old[q];
+  const int t = (int)dx.div((unsigned)i), ix = i - t * nx;
+  const int iz = (int)dy.div((unsigned)t), iy = t - iz * ny;
+  const bool inx[3] = {ix > 0, true, ix + 1 < nx}, iny[3] = {iy > 0, true, iy + 1 < ny},
+             inz[3] = {iz > 0, true, iz + 1 < nz};
+  double sum = 0.0;
+#pragma unroll
+  for (int k = 0; k < kSlots; ++k) {
+    const int sx = k % 3, sy = (k / 3) % 3, sz = k / 9;
+    const double xv =
+        inx[sx] && iny[sy] && inz[sz] ? __ldg(x + (i + ((sz - 1) * ny + (sy - 1)) * nx + (sx - 1))) : 0.0;
+    sum += a[k] * xv;
+  }
+  y[i] = sum;
+}
+
 // dst[i] = src[idx[i]]
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_gather(T* __restrict__ dst, const T* __restrict__ src,
@@ -847,6 +929,50 @@ __global__ void __launch_bounds__(kThreads) k_dot(int n, const double* __restric
   }
 }
 
+// A lone reduction of the vector routines in one launch: the block that arrives
+// last sums the partials as k_finalize does (same order, same bits) and stores
+// the result in host-mapped memory, behind it the call's number. count wraps to 0.
+struct LoneResult {
+  double value;
+  unsigned long long call;
+};
+template <bool MAX>
+__global__ void __launch_bounds__(kThreads) k_lone(int n, const double* __restrict__ x, const double* __restrict__ y,
+                                                   double* __restrict__ partials, unsigned* count,
+                                                   volatile LoneResult* out, unsigned long long call) {
+  __shared__ bool last;
+  const int stride = gridDim.x * blockDim.x;
+  double acc = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    if (MAX) {
+      const double d = fabs(x[i] - y[i]);
+      if (d > acc) acc = d;
+    } else {
+      acc += x[i] * y[i];
+    }
+  }
+  const double s = MAX ? block_max(acc) : block_sum(acc);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = s;
+    __threadfence();
+    last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  acc = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
+    const double p = __ldcg(partials + i);
+    acc = MAX ? fmax(acc, p) : acc + p;
+  }
+  const double r = MAX ? block_max(acc) : block_sum(acc);
+  if (threadIdx.x == 0) {
+    out->value = r;
+    __threadfence_system();
+    out->call = call;
+  }
+}
+
 // Flexible-CG step of the mixed form: z = widen(x32) together with the partials
 // of r'z (and of r'zprev for TWO) in k_dot<TWO>'s layout and order, so the
 // conversion pass and the copy of z into zprev go away (z and zprev are two
@@ -871,19 +997,6 @@ __global__ void __launch_bounds__(kThreads) k_widen_dot(int n, const float* __re
     const double s2 = block_sum(acc2);
     if (threadIdx.x == 0) partials[gridDim.x + blockIdx.x] = s2;
   }
-}
-
-// partial maxima of |v1 - v2| (ComputeResidual.cpp:70-75)
-__global__ void __launch_bounds__(kThreads) k_maxdiff(int n, const double* __restrict__ a,
-                                                      const double* __restrict__ b, double* __restrict__ partials) {
-  const int stride = gridDim.x * blockDim.x;
-  double m = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const double d = fabs(a[i] - b[i]);
-    if (d > m) m = d;
-  }
-  const double s = block_max(m);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
 // ---- CG scalar bookkeeping on the device -----------------------------------
@@ -931,6 +1044,24 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const double* __restrict_
   const double sum2 = op == kFinFlex ? block_sum(acc2) : 0.0;
   if (threadIdx.x != 0) return;
   apply_fin(op, sum, sum2, s, out);
+}
+
+// The same for kWideParts partials (the post-smoother's r'z slots, most of them
+// zero), sixteen to a thread, all requested at once: 64 dependent rounds of a
+// 256-thread block took 12.8 us of each CG iteration, this 3.8.
+constexpr int kWideParts = kColours * kDotStride, kWideThreads = 1024;
+__global__ void __launch_bounds__(kWideThreads) k_finalize_wide(const double* __restrict__ partials, int op,
+                                                                Scalars* s, double* out) {
+  static_assert(kWideParts == 16 * kWideThreads, "eight pairs a thread");
+  const double2* p = reinterpret_cast<const double2*>(partials) + threadIdx.x;
+  double2 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = p[i * kWideThreads];
+  double acc = 0.0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc += v[i].x + v[i].y;
+  const double sum = block_sum(acc);
+  if (threadIdx.x == 0) apply_fin(op, sum, 0.0, s, out);
 }
 
 // The ranks' values of one reduction, combined in rank order (a sum, or the
@@ -1040,6 +1171,30 @@ __global__ void __launch_bounds__(kThreads) k_adjoint_values(ColourGrid g, const
       const int c = col[mat_index<double>(k, q, pitch)];
       o[k] = c == n ? 0.0 : -(l * x[c]);
     }
+  }
+}
+
+// The same for a level whose columns follow from the grid, on natural-order
+// vectors: one thread per output, so the 27 n values, which are nearly all the
+// bytes there are, leave as whole lines (a thread per row stored 27 values 216
+// bytes apart: 128^3 783 us against 137).
+__global__ void __launch_bounds__(kThreads) k_adjoint_values_geo(int nx, int ny, int nz, FastDiv dx, FastDiv dy,
+                                                                 const double* __restrict__ lam,
+                                                                 const double* __restrict__ x,
+                                                                 double* __restrict__ out) {
+  const int n = nx * ny * nz;
+  const int rows = 1 << 10;  // rows of a block: its 27 * rows outputs
+  const int r0 = blockIdx.x * rows;
+  const int cnt = min(rows, n - r0) * kSlots;
+  double* o = out + (int64_t)r0 * kSlots;
+  for (int e = threadIdx.x; e < cnt; e += kThreads) {
+    const int row = e / kSlots, k = e - row * kSlots, i = r0 + row;
+    const int t = (int)dx.div((unsigned)i), ix = i - t * nx;
+    const int iz = (int)dy.div((unsigned)t), iy = t - iz * ny;
+    const int sz = k / 9 - 1, sy = k / 3 % 3 - 1, sx = k % 3 - 1;
+    const bool in = (unsigned)(ix + sx) < (unsigned)nx && (unsigned)(iy + sy) < (unsigned)ny &&
+                    (unsigned)(iz + sz) < (unsigned)nz;
+    o[e] = in ? -(__ldg(lam + i) * __ldg(x + (i + (sz * ny + sy) * nx + sx))) : 0.0;
   }
 }
 
