@@ -8,7 +8,9 @@
 #pragma once
 
 #include "bulk.cuh"
+#include "geo.cuh"
 #include "reduce.cuh"
+#include "tail.cuh"
 
 namespace hb {
 
@@ -236,6 +238,207 @@ __global__ void __launch_bounds__(MultiShape<LANES, PW>::threads, 1)
   }
 }
 
+// ---- form 3: columns from the grid (geo.cuh) ------------------------------------
+// The same sums with no columns read. Rows [r0, r1) of the colour block geo.
+// What bounds these kernels is the latency of the gathers (27 runs of 8 K bytes a
+// row), so each takes the most warps a SM holds: two systems a thread, 56
+// registers and two blocks of 16 consumer warps in the bulk-copy kernels (128^3,
+// eight systems: a phase 39 us, with four systems a thread and one block 48, the
+// SpMV 233 against 283), four systems a thread and five blocks of 8 in the register
+// kernels (first sweep 257 us; all of a row's values requested ahead, two blocks,
+// 374). Sweeps run in chunks of z pairs that keep x in the L2 were no faster.
+template <int K>
+__host__ __device__ constexpr int multi_lanes() {
+  return K / 2;
+}
+template <int K>
+__host__ __device__ constexpr int multi_first_lanes() {
+  return K >= 8 ? 2 : 1;
+}
+template <int K>
+using MultiGeo = BulkShape<double, K == 8 ? 1 : 2, 2, multi_lanes<K>(), kPackGeo>;
+
+// A full-slot phase.
+template <int K>
+__global__ void __launch_bounds__(MultiGeo<K>::threads, 2)
+    k_gs_phase_m_geo(const double* __restrict__ val, int64_t pitch, const double* __restrict__ rhs, double* x, int r0,
+                     int r1, unsigned* fault, const __grid_constant__ CUtensorMap tm_val, int sink,
+                     const __grid_constant__ GeoPhase geo) {
+  constexpr int LANES = multi_lanes<K>(), S = K / LANES;
+  const int a0 = r0 & ~(kBulkRows - 1);
+  const int ntiles = (r1 - a0 + kBulkRows - 1) / kBulkRows;
+  bulk_tiles<double, MultiGeo<K>>(
+      val, nullptr, pitch, ntiles, [&](int tile) { return a0 + (int64_t)tile * kBulkRows; },
+      [&](int64_t q0, const double* sv, const int*, int t) {
+        const int row = t / LANES;
+        const int off = (t % LANES) * S;
+        const int q = (int)q0 + row;
+        if (q < r0 || q >= r1) return;
+        const GeoRow g(geo, q);
+        double sum[S], xd[S];
+        load_k<S>(rhs + (int64_t)q * K + off, sum);
+#pragma unroll
+        for (int j = 0; j < S; ++j) xd[j] = 0.0;
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k) {
+          const double a = sv[k * kBulkRows + row];
+          double xv[S];
+          load_k<S>(x + (int64_t)g.col(geo, k, sink) * K + off, xv);
+#pragma unroll
+          for (int j = 0; j < S; ++j) {
+            sum[j] -= a * xv[j];
+            if (k == kDiagSlot) xd[j] = xv[j];
+          }
+        }
+        const double d = sv[kDiagSlot * kBulkRows + row];
+        double out[S];
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+          sum[j] += xd[j] * d;
+          out[j] = sum[j] / d;
+        }
+        store_k<S>(x + (int64_t)q * K + off, out);
+      },
+      fault, tm_val, tm_val);
+}
+
+// A first-sweep phase.
+template <int K>
+__global__ void __launch_bounds__(kThreads, 5)
+    k_gs_first_m_geo(const double* __restrict__ val, int64_t pitch, const double* __restrict__ rhs, double* x, int r0,
+                     int r1, uint32_t mask, int sink, const __grid_constant__ GeoPhase geo) {
+  constexpr int LANES = multi_first_lanes<K>(), S = K / LANES;
+  const int64_t work = (int64_t)(r1 - r0) * LANES;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < work; t += stride) {
+    const int q = r0 + (int)(t / LANES);
+    const int off = (int)(t % LANES) * S;
+    const double d = __ldg(val + kDiagSlot * pitch + q);
+    double sum[S];
+    load_k<S>(rhs + (int64_t)q * K + off, sum);
+    const GeoRow g(geo, q);
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k) {
+      if (mask & (1u << k)) {
+        const double a = __ldg(val + k * pitch + q);
+        double xv[S];
+        load_k<S>(x + (int64_t)g.col(geo, k, sink) * K + off, xv);
+#pragma unroll
+        for (int j = 0; j < S; ++j) sum[j] -= a * xv[j];
+      }
+    }
+    double out[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) out[j] = sum[j] / d;
+    store_k<S>(x + (int64_t)q * K + off, out);
+  }
+}
+
+// y = A x; SLAB: tiles of one z pair in all eight colours, then the next (the
+// host checks that its runs are whole tiles), so that the K systems' x comes
+// from memory once. DOT as k_spmv_m.
+template <int K, bool DOT, bool SLAB>
+__global__ void __launch_bounds__(MultiGeo<K>::threads, 2)
+    k_spmv_m_geo(const double* __restrict__ val, int64_t pitch, const double* __restrict__ x,
+                 double* __restrict__ y, int n, int per, double* __restrict__ partials, unsigned* fault,
+                 const __grid_constant__ CUtensorMap tm_val, int sink, const __grid_constant__ GeoGrid geo) {
+  constexpr int LANES = multi_lanes<K>(), S = K / LANES;
+  __shared__ GeoPhase blocks[kColours];
+  for (int i = threadIdx.x; i < (int)(sizeof(blocks) / sizeof(int)); i += blockDim.x)
+    reinterpret_cast<int*>(blocks)[i] = reinterpret_cast<const int*>(geo.block)[i];
+  const int off = (int)(threadIdx.x % LANES) * S;  // the producer warp (32 threads) keeps the lanes aligned
+  double acc[S];
+#pragma unroll
+  for (int j = 0; j < S; ++j) acc[j] = 0.0;
+  const int ntiles = (n + kBulkRows - 1) / kBulkRows;
+  bulk_tiles<double, MultiGeo<K>>(
+      val, nullptr, pitch, ntiles,
+      [&](int tile) -> int64_t {
+        const int t = tile * kBulkRows;
+        if (!SLAB) return t;
+        const int h = t / (kColours * per), rem = t - h * kColours * per, s = rem / per;  // per: rows of a colour in a z pair
+        return geo.block[s].start + h * per + (rem - s * per);
+      },
+      [&](int64_t q0, const double* sv, const int*, int t) {
+        const int row = t / LANES;
+        const int q = (int)q0 + row;
+        if (q >= n) return;
+        int at = 0;
+#pragma unroll
+        for (int s = 1; s < kColours; ++s) at += q >= geo.block[s].start ? 1 : 0;
+        const GeoPhase& b = blocks[at];
+        const GeoRow g(b, q);
+        double sum[S], xq[S];
+#pragma unroll
+        for (int j = 0; j < S; ++j) sum[j] = xq[j] = 0.0;
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k) {
+          const double a = sv[k * kBulkRows + row];
+          double xv[S];
+          load_k<S>(x + (int64_t)g.col(b, k, sink) * K + off, xv);
+#pragma unroll
+          for (int j = 0; j < S; ++j) {
+            sum[j] += a * xv[j];
+            if (k == kDiagSlot) xq[j] = xv[j];
+          }
+        }
+        store_k<S>(y + (int64_t)q * K + off, sum);
+        if (DOT) {
+#pragma unroll
+          for (int j = 0; j < S; ++j) acc[j] += xq[j] * sum[j];
+        }
+      },
+      fault, tm_val, tm_val);
+  if (DOT) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const double s = block_sum(off == (j / S) * S ? acc[j % S] : 0.0);
+      if (threadIdx.x == 0) partials[j * gridDim.x + blockIdx.x] = s;
+    }
+  }
+}
+
+// Residual at the injected rows r0 .. r0 + nc, the all-even points.
+template <int K>
+__global__ void __launch_bounds__(kThreads, 5)
+    k_restrict_m_geo(const double* __restrict__ val, int64_t pitch, const double* __restrict__ rf,
+                     const double* __restrict__ xf, const int* __restrict__ tq, double* __restrict__ rc, int r0,
+                     int nc, int sink, const __grid_constant__ GeoPhase geo) {
+  constexpr int LANES = multi_first_lanes<K>(), S = K / LANES;
+  const int64_t work = (int64_t)nc * LANES;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < work; w += stride) {
+    const int t = (int)(w / LANES);
+    const int off = (int)(w % LANES) * S;
+    const int f = r0 + t;
+    const GeoRow g(geo, f);
+    double sum[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) sum[j] = 0.0;
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k) {
+      const double a = __ldg(val + k * pitch + f);
+      double xv[S];
+      load_k<S>(xf + (int64_t)g.col(geo, k, sink) * K + off, xv);
+#pragma unroll
+      for (int j = 0; j < S; ++j) sum[j] += a * xv[j];
+    }
+    double r[S], out[S];
+    load_k<S>(rf + (int64_t)f * K + off, r);
+#pragma unroll
+    for (int j = 0; j < S; ++j) out[j] = r[j] - sum[j];
+    store_k<S>(rc + (int64_t)tq[t] * K + off, out);
+  }
+}
+
+// The small levels (tail.cuh): cluster j of the grid runs system j's.
+template <int K>
+__global__ void __launch_bounds__(kTailThreads, 1)
+    k_tail_m(const __grid_constant__ TailDesc<double> D, const double* __restrict__ rhs, double* x, unsigned* fault) {
+  const int j = (int)(blockIdx.x / cluster_blocks());
+  tail_run<double, K>(D, rhs + j, x + j, false, fault, j);
+}
+
 // rc = (rf - A xf) at the injected rows (sorted transfer pairs), K systems; LANES as in k_gs_phase_m.
 template <int K, int LANES>
 __global__ void __launch_bounds__(kThreads) k_restrict_m(const double* __restrict__ val, const int* __restrict__ col,
@@ -422,20 +625,27 @@ __global__ void __launch_bounds__(kThreads) k_update_xr_m(double* __restrict__ x
 
 enum MFinOp : int { kMNorm0 = 0, kMRtzFirst = 1, kMRtz = 2, kMPap = 3, kMNormr = 4 };
 
-// One block: fixed-order reduction of the K partial sets, then the scalar step of
-// `op` for every system (the single-system rules of CG.cpp:96-124, per system).
+// Fixed-order reduction of the K partial sets, then the scalar step of `op` for
+// every system (the single-system rules of CG.cpp:96-124, per system): one block
+// for each system.
 template <int K>
 __global__ void __launch_bounds__(kThreads) k_finalize_m(const double* __restrict__ partials, int nparts, int op,
                                                          MScalars* s, int iter, double tol) {
   double sum[K];
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
+  {
+    const int j = blockIdx.x;
     double acc = 0.0;
+#pragma unroll 4
     for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc += partials[j * nparts + i];
-    sum[j] = block_sum(acc);
+    const double v = block_sum(acc);
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      if (i == j) sum[i] = v;
   }
   if (threadIdx.x != 0) return;
+#pragma unroll
   for (int j = 0; j < K; ++j) {
+    if (j != (int)blockIdx.x) continue;
     switch (op) {
       case kMNorm0: {
         s->normr2[j] = sum[j];

@@ -225,10 +225,13 @@ struct TailSlab {
 // to a row, the sum passed between them, 1.2 us.
 // A forward phase of a sweep from zero loads only its masked slots' values and
 // takes zero for the others: their products are +0, which change no sum.
-template <typename T, bool ZERO>
+// ST: entries from one row's right-hand side or solution to the next's (the
+// systems of a multi-system solve interleave), off: the system.
+template <typename T, bool ZERO, int ST>
 __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem, const TailPhase* __restrict__ phases,
                                            const TailRow* __restrict__ table, int rank, const T* __restrict__ rhs,
-                                           T* xg, bool keep, bool restrict_, bool prolong, TailWait& wait) {
+                                           T* xg, bool keep, bool restrict_, bool prolong, TailWait& wait,
+                                           int off) {
   const TailLevel<T>& L = D.lev[l];
   if (rank >= L.act) {
     cluster_sync_all();
@@ -279,11 +282,11 @@ __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem,
     const TailPhase PI = tab[7];
     for (int u = tid; u < PI.cnt; u += kTailThreads) {
       const unsigned t = table[PI.t0 + u];
-      put(t, S.xs[t & ~(kTailLow | kTailHigh)] + __ldcg(C.x + S.coarse(D, C, PI, u)));
+      put(t, S.xs[t & ~(kTailLow | kTailHigh)] + __ldcg(C.x + (int64_t)S.coarse(D, C, PI, u) * ST + off));
     }
     wait.end(rank, L.act, PI.sent);
   }
-  va[kSlots] = __ldcg(rhs + P.q0 + (i < P.cnt ? i : 0));
+  va[kSlots] = __ldcg(rhs + (int64_t)(P.q0 + (i < P.cnt ? i : 0)) * ST);
   // one row of this thread, its values in a; false after the last
   auto step = [&](const T(&a)[kSlots + 1], T(&next)[kSlots + 1]) -> bool {
     // the next row: the phase's next chunk, or the next phase's first (a thread
@@ -299,7 +302,7 @@ __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem,
       const int nc = ni < NP.cnt ? ni : 0;
       NR = table[NP.t0 + nc];
       fetch(next, NP.q0 + nc, NP, nj);
-      next[kSlots] = __ldcg(rhs + NP.q0 + nc);
+      next[kSlots] = __ldcg(rhs + (int64_t)(NP.q0 + nc) * ST);
     }
     const bool res = j == 15;  // the residual at the injected rows
     if (i < P.cnt) {
@@ -320,13 +323,13 @@ __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem,
       for (int k = 0; k < kSlots; ++k) sum -= a[k] * xv[k];
       if (res) {
         const TailLevel<T>& C = D.lev[l + 1];
-        C.r[S.coarse(D, C, P, i)] = rv + sum;  // sum: minus the row's product
+        C.r[(int64_t)S.coarse(D, C, P, i) * ST + off] = rv + sum;  // sum: minus the row's product
       } else {
         const T d = a[kDiagSlot];
         if (!(ZERO && j < 8)) sum += xv[kDiagSlot] * d;
         const T out = sum / d;
         put(R, out);
-        if (keep && j >= 7) xg[P.q0 + i] = out;
+        if (keep && j >= 7) xg[(int64_t)(P.q0 + i) * ST] = out;
       }
     }
     if (!same && !res) wait.end(rank, L.act, P.sent);
@@ -341,10 +344,11 @@ __device__ __forceinline__ void tail_sweep(const TailDesc<T>& D, int l, T* smem,
 }
 
 // The V-cycle of a problem's levels from D.lev[0] down (rhs, x: level D.lev[0]'s
-// vectors), or with `step` one symmetric step on x with right-hand side rhs.
-template <typename T>
+// vectors, at the system's first entry), or with `step` one symmetric step on x
+// with right-hand side rhs.
+template <typename T, int ST = 1>
 __device__ __forceinline__ void tail_run(const TailDesc<T>& D, const T* __restrict__ rhs, T* x, bool step,
-                                         unsigned* fault) {
+                                         unsigned* fault, int off = 0) {
   extern __shared__ __align__(16) unsigned char tail_smem[];
   __shared__ TailSync sync;
   __shared__ TailPhase phases[kMaxLevels * kColours];
@@ -382,19 +386,19 @@ __device__ __forceinline__ void tail_run(const TailDesc<T>& D, const T* __restri
         const int c = (ix & 1) | ((iy & 1) << 1) | ((iz & 1) << 2);
         const int cx = ColourGrid::half(L.nx, c & 1), cy = ColourGrid::half(L.ny, (c >> 1) & 1);
         S.xs[lz * S.sh.sz + (iy + 1) * S.sh.sy + (ix & 1) * S.sh.hx + (ix >> 1) + 1] =
-            __ldcg(x + L.start[D.pos[c]] + ((iz >> 1) * cy + (iy >> 1)) * cx + (ix >> 1));
+            __ldcg(x + (int64_t)(L.start[D.pos[c]] + ((iz >> 1) * cy + (iy >> 1)) * cx + (ix >> 1)) * ST);
       }
     }
-    tail_sweep<T, false>(D, 0, smem, phases, table, rank, rhs, x, true, false, false, wait);
+    tail_sweep<T, false, ST>(D, 0, smem, phases, table, rank, rhs, x, true, false, false, wait, off);
     cluster_sync_relaxed();
     return;
   }
   for (int l = 0; l < D.nlev; ++l)
-    tail_sweep<T, true>(D, l, smem, phases, table, rank, l == 0 ? rhs : D.lev[l].r, l == 0 ? x : D.lev[l].x, l + 1 == D.nlev,
-                        l + 1 < D.nlev, false, wait);
+    tail_sweep<T, true, ST>(D, l, smem, phases, table, rank, l == 0 ? rhs : D.lev[l].r + off,
+                            l == 0 ? x : D.lev[l].x + off, l + 1 == D.nlev, l + 1 < D.nlev, false, wait, off);
   for (int l = D.nlev - 2; l >= 0; --l)
-    tail_sweep<T, false>(D, l, smem, phases, table, rank, l == 0 ? rhs : D.lev[l].r, l == 0 ? x : D.lev[l].x, true, false, true,
-                         wait);
+    tail_sweep<T, false, ST>(D, l, smem, phases, table, rank, l == 0 ? rhs : D.lev[l].r + off,
+                             l == 0 ? x : D.lev[l].x + off, true, false, true, wait, off);
   cluster_sync_relaxed();
 }
 
