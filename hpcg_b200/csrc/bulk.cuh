@@ -342,6 +342,16 @@ __device__ __forceinline__ uint64_t evict_first_policy() {
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 
+// The wait, and the pointers to what the kernels before may have written made new
+// to the compiler: loads through a const __restrict__ pointer or __ldg are free to
+// move across any barrier, so a kernel that was launched early must not hold the
+// address before the wait.
+template <typename... P>
+__device__ __forceinline__ void griddep_wait_for(P&... p) {
+  griddep_wait();
+  ((void)([&] { asm volatile("" : "+l"(p)::"memory"); }()), ...);
+}
+
 __device__ __forceinline__ void record_fault(unsigned* fault, unsigned code) {
   *(volatile unsigned*)fault = code;
   __threadfence_system();

@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <thread>
 #include <utility>
@@ -446,6 +447,41 @@ inline void bulk_attr(Kern k, int smem, int device, std::atomic<uint64_t>* done)
   if (done->load(std::memory_order_acquire) & bit) return;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   done->fetch_or(bit, std::memory_order_release);
+}
+
+// Launches k on `stream` so that it may start while the kernel before it drains
+// (programmatic dependent launch); k must call griddep_wait before it reads or
+// writes what that kernel, or any before it, touches. Every kernel of such a
+// chain waits in at least one block, so one that has completed has all before it
+// completed too. HPCG_B200_PDL=0: plain launches. A refusal is tried plainly.
+inline bool pdl_enabled() {
+  static const bool on = [] {
+    const char* e = std::getenv("HPCG_B200_PDL");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_early(cudaStream_t stream, void (*k)(KArgs...), int grid, int threads, size_t smem,
+                         Args&&... args) {
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+  if (e != cudaSuccess && cfg.numAttrs) {
+    cudaGetLastError();
+    cfg.numAttrs = 0;
+    e = cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+  }
+  return e;
 }
 
 // problem handle validity

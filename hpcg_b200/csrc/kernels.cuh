@@ -323,6 +323,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) * R * __builtin_popcount(M
                    int sink, const __grid_constant__ GeoPhase geo) {
   const int tile = kThreads * R;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  griddep_launch_dependents();
+  bool waited = false;
   for (int b0 = r0 + blockIdx.x * tile; b0 < r1; b0 += gridDim.x * tile) {
     const int q0 = b0 + warp * 32 * R + lane;
     T a[R][kSlots], d[R], sum[R];
@@ -334,9 +336,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) * R * __builtin_popcount(M
         for (int k = 0; k < kSlots; ++k)
           if (MASK >> k & 1u) a[r][k] = __ldcs(val + mat_index<T>(k, q, pitch));
         d[r] = __ldcs(val + mat_index<T>(kDiagSlot, q, pitch));
-        sum[r] = (T)rhs[q];
       }
     }
+    if (!waited) {  // the first rows' values are on their way while the phase before drains
+      griddep_wait_for(rhs, x);
+      waited = true;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (q0 + 32 * r < r1) sum[r] = (T)rhs[q0 + 32 * r];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int q = q0 + 32 * r;
@@ -793,6 +801,8 @@ __global__ void __launch_bounds__(RestrictShape<T, PW>::threads, 1)
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_prolong(const int* __restrict__ tf, const int* __restrict__ tq,
                                                       const T* __restrict__ xc, T* __restrict__ xf, int nc) {
+  griddep_launch_dependents();
+  griddep_wait_for(xc, xf);
   const int stride = gridDim.x * blockDim.x;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nc; t += stride) xf[tf[t]] += xc[tq[t]];
 }
@@ -914,6 +924,8 @@ __global__ void __launch_bounds__(kThreads) k_waxpby(int n, double alpha, const 
 template <bool TWO>
 __global__ void __launch_bounds__(kThreads) k_dot(int n, const double* __restrict__ x, const double* __restrict__ y,
                                                   const double* __restrict__ y2, double* __restrict__ partials) {
+  griddep_launch_dependents();
+  griddep_wait_for(x, y, y2);
   const int stride = gridDim.x * blockDim.x;
   double acc = 0.0, acc2 = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -982,6 +994,8 @@ __global__ void __launch_bounds__(kThreads) k_widen_dot(int n, const float* __re
                                                         const double* __restrict__ r, double* __restrict__ z,
                                                         const double* __restrict__ zprev,
                                                         double* __restrict__ partials) {
+  griddep_launch_dependents();
+  griddep_wait_for(x32, r, z, zprev);
   const int stride = gridDim.x * blockDim.x;
   double acc = 0.0, acc2 = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -1030,6 +1044,8 @@ __device__ __forceinline__ void apply_fin(int op, double sum, double sum2, Scala
 // at partials[nparts..] for kFinFlex), then the scalar update of `op`.
 __global__ void __launch_bounds__(kThreads) k_finalize(const double* __restrict__ partials, int nparts, int op,
                                                        Scalars* s, double* out) {
+  griddep_launch_dependents();
+  griddep_wait_for(partials, s, out);
   double acc = 0.0, acc2 = 0.0;
   if (op == kFinMax) {
     for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc = fmax(acc, partials[i]);
@@ -1052,6 +1068,8 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const double* __restrict_
 constexpr int kWideParts = kColours * kDotStride, kWideThreads = 1024;
 __global__ void __launch_bounds__(kWideThreads) k_finalize_wide(const double* __restrict__ partials, int op,
                                                                 Scalars* s, double* out) {
+  griddep_launch_dependents();
+  griddep_wait_for(partials, s, out);
   static_assert(kWideParts == 16 * kWideThreads, "eight pairs a thread");
   const double2* p = reinterpret_cast<const double2*>(partials) + threadIdx.x;
   double2 v[8];
@@ -1082,6 +1100,8 @@ __global__ void k_finalize_ranks(const double* __restrict__ vals, int nvals, int
 // first (iteration 1): p = z (CG.cpp:109), x untouched.
 __device__ __forceinline__ void update_px(int n, const double* __restrict__ z, double* p, double* x,
                                           const Scalars* __restrict__ s, bool first) {
+  griddep_launch_dependents();
+  griddep_wait_for(z, p, x, s);
   const double beta = s->beta, alpha = s->alpha;
   const int stride = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -1110,6 +1130,8 @@ __global__ void __launch_bounds__(kThreads) k_update_px_iter(int n, const double
 __global__ void __launch_bounds__(kThreads) k_update_r(int n, double* r, const double* __restrict__ Ap,
                                                        const Scalars* __restrict__ s, double* __restrict__ partials,
                                                        float* __restrict__ r32 = nullptr) {
+  griddep_launch_dependents();
+  griddep_wait_for(r, Ap, s);
   const double malpha = -s->alpha;
   const int stride = gridDim.x * blockDim.x;
   double acc = 0.0;

@@ -88,10 +88,7 @@ bool gs_bulk_launch_p(Context* c, const Level& L, const T* val, const TR* rhs, T
   if (DOT && g > kDotStride) g = kDotStride;
   // programmatic dependent launch: the phase's producer streams its first
   // matrix tiles while the previous kernel finishes (HPCG_B200_PDL=0: off)
-  static const bool pdl = [] {
-    const char* e = std::getenv("HPCG_B200_PDL");
-    return !(e && e[0] == '0');
-  }();
+  const bool pdl = pdl_enabled();
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(g);
@@ -232,8 +229,8 @@ void gs_first_geo_at(Context* c, const Level& L, const T* val, const TR* rhs, T*
   if (r1 <= r0) return;
   auto k = k_gs_first_geo<T, TR, first_mask_default(S), R>;
   const int64_t units = ((int64_t)r1 - r0 + R - 1) / R;
-  k<<<grid_of(c, k, units), kThreads, 0, c->stream>>>(val, L.pitch, rhs, x, r0, r1, sink_of(L),
-                                                   L.geo_cols->block[S]);
+  launch_early(c->stream, k, grid_of(c, k, units), kThreads, 0, val, L.pitch, rhs, x, r0, r1, sink_of(L),
+               L.geo_cols->block[S]);
 }
 template <typename T, typename TR, int R>
 void gs_first_geo(Context* c, const Level& L, const T* val, const TR* rhs, T* x, int r0, int r1, int s) {
@@ -322,8 +319,8 @@ int spmv_bulk_launch(Context* c, const Level& L, const T* val, const T* x, T* y,
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)c->sms));
   static const GeoGrid none{};
   const GeoGrid& geo = PW == kPackGeo ? *L.geo_cols : none;
-  k<<<g, Shape::threads, smem, c->stream>>>(L.g, val, cols_of<T>(L), L.pitch, x, y, L.n, partials, c->fault, m->val,
-                                            m->col, (const unsigned char*)L.colp, sink_of(L), geo);
+  launch_early(c->stream, k, g, Shape::threads, smem, L.g, val, cols_of<T>(L), L.pitch, x, y, L.n, partials, c->fault,
+               m->val, m->col, (const unsigned char*)L.colp, sink_of(L), geo);
   return g;
 }
 
@@ -409,8 +406,8 @@ bool restrict_bulk_p(Context* c, const Level& L, const T* val, const T* rf, cons
   const int g = (int)std::min<int64_t>(tiles, (int64_t)c->sms);
   GeoPhase geo{};
   if constexpr (PW == kPackGeo) geo = L.geo_cols->block[sweep_at(L, L.tf_run)];
-  k<<<g, Shape::threads, smem, c->stream>>>(val, cols_of<T>(L), L.pitch, rf, xf, L.tq, rc, L.tf_run, nc, c->fault,
-                                            *tv, *tc, (const unsigned char*)L.colp, sink_of(L), geo);
+  launch_early(c->stream, k, g, Shape::threads, smem, val, cols_of<T>(L), L.pitch, rf, xf, L.tq, rc, L.tf_run, nc,
+               c->fault, *tv, *tc, (const unsigned char*)L.colp, sink_of(L), geo);
   return true;
 }
 
@@ -716,8 +713,8 @@ int mg_level(hpcg_b200_problem* p, int l, const double* r, double* x, double* rt
     HB_CK(cudaGetLastError());
     HB_TRY(prof_end(c, l == 0 ? kProfRestrict : -1, ev0, C.n));
     HB_TRY(l == 0 ? coarse_vcycle(p, false) : mg_level(p, l + 1, C.r, C.x));
-    k_prolong<double><<<grid_for(c, C.n, kThreads, kPerSm), kThreads, 0, c->stream>>>(L.tf, L.tq, C.x, x, C.n);
-    HB_CK(cudaGetLastError());
+    HB_CK(launch_early(c->stream, k_prolong<double>, grid_for(c, C.n, kThreads, kPerSm), kThreads, 0, L.tf, L.tq, C.x,
+                       x, C.n));
     if (rtz) HB_CK(cudaMemsetAsync(rtz, 0, sizeof(double) * kColours * kDotStride, c->stream));
     HB_TRY(symgs_level(p, l, r, x, false, rtz));
   }
@@ -1012,10 +1009,9 @@ int autotune(hpcg_b200_problem* P) {
 
 int finalize(Context* c, int nparts, int op, double* out = nullptr) {
   if (nparts == kWideParts && op != kFinMax && op != kFinFlex)
-    k_finalize_wide<<<1, kWideThreads, 0, c->stream>>>(c->partials, op, c->scal, out);
+    HB_CK(launch_early(c->stream, k_finalize_wide, 1, kWideThreads, 0, c->partials, op, c->scal, out));
   else
-    k_finalize<<<1, kThreads, 0, c->stream>>>(c->partials, nparts, op, c->scal, out);
-  HB_CK(cudaGetLastError());
+    HB_CK(launch_early(c->stream, k_finalize, 1, kThreads, 0, c->partials, nparts, op, c->scal, out));
   return HPCG_B200_OK;
 }
 
@@ -1129,17 +1125,15 @@ int cg_iteration_body(hpcg_b200_problem* P, bool prec) {
     } else {
       HB_CK(cudaMemcpyAsync(P->z, P->r, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
     }
-    k_dot<false><<<nb, kThreads, 0, c->stream>>>(n, P->r, P->z, nullptr, c->partials);
-    HB_CK(cudaGetLastError());
+    HB_CK(launch_early(c->stream, k_dot<false>, nb, kThreads, 0, n, P->r, P->z, nullptr, c->partials));
     HB_TRY(finalize(c, nb, kFinRtzIter));
   }
-  k_update_px_iter<<<gv, kThreads, 0, c->stream>>>(n, P->z, P->p, P->x, c->scal);  // with x of the last iteration
-  HB_CK(cudaGetLastError());
+  // with x of the last iteration
+  HB_CK(launch_early(c->stream, k_update_px_iter, gv, kThreads, 0, n, P->z, P->p, P->x, c->scal));
   const int gs = spmv_dispatch<double, true>(c, L, L.val, P->p, P->Ap, c->partials);
   HB_CK(cudaGetLastError());
   HB_TRY(finalize(c, gs, kFinPap));
-  k_update_r<<<nb, kThreads, 0, c->stream>>>(n, P->r, P->Ap, c->scal, c->partials);
-  HB_CK(cudaGetLastError());
+  HB_CK(launch_early(c->stream, k_update_r, nb, kThreads, 0, n, P->r, P->Ap, c->scal, c->partials, nullptr));
   return finalize(c, nb, kFinNormr);
 }
 
@@ -1457,8 +1451,8 @@ int mg32_level(hpcg_b200_problem* p, int l, const float* r, float* x) {
     restrict_dispatch<float>(c, L, L.val32, r, x, C.r32, C.n);
     HB_CK(cudaGetLastError());
     HB_TRY(l == 0 ? coarse_vcycle(p, true) : mg32_level(p, l + 1, C.r32, C.x32));
-    k_prolong<float><<<grid_for(c, C.n, kThreads, kPerSm), kThreads, 0, c->stream>>>(L.tf, L.tq, C.x32, x, C.n);
-    HB_CK(cudaGetLastError());
+    HB_CK(launch_early(c->stream, k_prolong<float>, grid_for(c, C.n, kThreads, kPerSm), kThreads, 0, L.tf, L.tq, C.x32,
+                       x, C.n));
     HB_TRY((gs_colour<float, float>(c, L, L.val32, r, x, false, l == 0)));
   }
   return HPCG_B200_OK;
@@ -1498,18 +1492,16 @@ int run_cg_mixed(hpcg_b200_problem* P, int max_iter, double tol, int* niters, do
       HB_TRY(finalize(c, nb, kFinRtzFirst));
       HB_CK(cudaMemcpyAsync(P->p, zc, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
     } else {
-      k_widen_dot<true><<<nb, kThreads, 0, c->stream>>>(n, L.x32, P->r, zc, zp, c->partials);
-      HB_CK(cudaGetLastError());
+      HB_CK(launch_early(c->stream, k_widen_dot<true>, nb, kThreads, 0, n, L.x32, P->r, zc, zp, c->partials));
       HB_TRY(finalize(c, nb, kFinFlex));
-      k_update_px<<<gv, kThreads, 0, c->stream>>>(n, zc, P->p, P->x, c->scal);  // with x of iteration k - 1
-      HB_CK(cudaGetLastError());
+      // with x of iteration k - 1
+      HB_CK(launch_early(c->stream, k_update_px, gv, kThreads, 0, n, zc, P->p, P->x, c->scal));
     }
     std::swap(zc, zp);
     const int gs = spmv_dispatch<double, true>(c, L, L.val, P->p, P->Ap, c->partials);
     HB_CK(cudaGetLastError());
     HB_TRY(finalize(c, gs, kFinPap));
-    k_update_r<<<nb, kThreads, 0, c->stream>>>(n, P->r, P->Ap, c->scal, c->partials, L.r32);
-    HB_CK(cudaGetLastError());
+    HB_CK(launch_early(c->stream, k_update_r, nb, kThreads, 0, n, P->r, P->Ap, c->scal, c->partials, L.r32));
     HB_TRY(finalize(c, nb, kFinNormr));
     HB_TRY(read_scalars(c));
     normr = std::sqrt(c->scal_host->normr2);

@@ -153,13 +153,15 @@ bool launch(hpcg_b200_problem* p, int l, int nlev, const T* rhs, T* x, bool step
   cfg.blockDim = dim3(kTailThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = c->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = size;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, k, D, rhs, x, step ? 1 : 0, c->fault);
   if (e != cudaSuccess) {
     set_error("k_tail", e);

@@ -356,6 +356,7 @@ __device__ __forceinline__ void tail_run(const TailDesc<T>& D, const T* __restri
   TailRow* table = reinterpret_cast<TailRow*>(smem + D.elems);
   const int rank = (int)cluster_rank();
   TailWait wait{&sync, fault, 0, 0u, false};
+  griddep_launch_dependents();
   if (threadIdx.x == 0) {
     mbar_init(&sync.bar[0], 1);
     mbar_init(&sync.bar[1], 1);
@@ -374,6 +375,7 @@ __device__ __forceinline__ void tail_run(const TailDesc<T>& D, const T* __restri
     const TailPhase P = phases[u];
     for (int i = threadIdx.x; i < P.cnt; i += kTailThreads) table[P.t0 + i] = S.row(P, i);
   }
+  griddep_wait();  // (above: this block's own memory and the launch's description only)
   if (step) {
     const TailLevel<T>& L = D.lev[0];
     if (rank < L.act) {
