@@ -48,10 +48,10 @@ namespace hb {
 constexpr int kConfigs = 8;     // configurations of the SpMV and the restriction
 constexpr int kBulkMvCfg = 7;   // the SpMV through the bulk-copy pipeline (k_spmv_bulk)
 constexpr int kGsConfigs = 13;  // configurations of the Gauss-Seidel phases
-constexpr int kGsFull = 11;     // of which run a phase of all slots (the others: first-sweep phases only)
+constexpr int kGsFull = 12;     // of which run a phase of all slots (the others: first-sweep phases only)
 constexpr int kTileCfg = 9;     // the tiled configuration
 constexpr int kBulkCfg = 10;    // the bulk-copy pipeline
-constexpr int kGeoCfg = 11;     // and the next: columns from the grid, 1 or 2 rows a thread (k_gs_first_geo)
+constexpr int kGeoCfg = 11;     // and the next: columns from the grid, 1 or 2 rows a thread (k_gs_first_geo, k_gs_geo)
 // configurations without a row-alignment requirement that run their own kernels
 __host__ __device__ constexpr bool cfg_tiled(int cfg) { return cfg >= kTileCfg; }
 __host__ __device__ constexpr int cfg_sched(int cfg) { return cfg == 2 || cfg == 3 ? kStaged : kPlain; }
@@ -362,6 +362,55 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) * R * __builtin_popcount(M
         x[q] = sum[r] / d[r];
       }
     }
+  }
+}
+
+// Full-slot phase with the columns from the grid, one row a thread
+// (configuration 11): for phases of one or two rounds of blocks on the SMs. Such
+// a phase is a launch and a chain of latencies, not a stream: every row's 27
+// values are requested before the wait for the phase before, so that what is left
+// behind it is the gathers, the sum, the division and the store. Two blocks an SM
+// (126 registers) keep the 27 values and the 27 gathers of a row in flight. The
+// bulk-copy pipeline sets up its barriers and starts its copies inside the phase:
+// a phase of 64^3 took 3.9 us with it and takes 3.4, of 80^3 5.2 and 4.1, of
+// 104^3 8.1 and 7.5, of 128^3 (3.5 rounds) 12.1 and 13.3.
+// DOT: also block partials of sum_i rhs_i * x_i, as k_gs_phase.
+template <typename T, typename TR, bool DOT>
+__global__ void __launch_bounds__(kThreads, 2)
+    k_gs_geo(const T* __restrict__ val, int64_t pitch, const TR* __restrict__ rhs, T* x, int r0, int r1, int sink,
+             double* __restrict__ dot, const __grid_constant__ GeoPhase geo) {
+  griddep_launch_dependents();
+  bool waited = false;
+  double acc = 0.0;
+  for (int b0 = r0 + blockIdx.x * kThreads; b0 < r1; b0 += gridDim.x * kThreads) {
+    const int q = b0 + threadIdx.x;
+    T a[kSlots];
+    if (q < r1) {
+#pragma unroll
+      for (int k = 0; k < kSlots; ++k) a[k] = __ldg(val + mat_index<T>(k, q, pitch));
+    }
+    if (!waited) {
+      griddep_wait_for(rhs, x);
+      waited = true;
+    }
+    if (q < r1) {
+      const GeoRow g(geo, q);
+      const T rv = (T)rhs[q];
+      T xv[kSlots];
+#pragma unroll
+      for (int k = 0; k < kSlots; ++k) xv[k] = __ldg(x + g.col(geo, k, sink));
+      T sum = rv;
+#pragma unroll
+      for (int k = 0; k < kSlots; ++k) sum -= a[k] * xv[k];
+      sum += xv[kDiagSlot] * a[kDiagSlot];
+      const T out = sum / a[kDiagSlot];
+      x[q] = out;
+      if (DOT) acc += (double)rv * (double)out;
+    }
+  }
+  if (DOT) {
+    const double s = block_sum(acc);
+    if (threadIdx.x == 0) dot[blockIdx.x] = s;
   }
 }
 

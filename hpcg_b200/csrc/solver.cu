@@ -185,13 +185,36 @@ void gs_launch(Context* c, const Level& L, const T* val, const TR* rhs, T* x, in
 // on a multiple of R (vector loads); otherwise the scalar configuration 1 runs.
 // Interleaved rows need no alignment.
 inline int usable_cfg(int cfg, int r0) {
-  if (cfg >= kGeoCfg) return kBulkCfg;  // (first-sweep phases only, see gs_first_dispatch)
+  if (cfg >= kGeoCfg) return kBulkCfg;  // (no columns from the grid: see gs_dispatch, gs_first_dispatch)
   return cfg_tiled(cfg) || cfg_interleaved(cfg) || r0 % cfg_rows(cfg) == 0 ? cfg : 1;
+}
+
+// k_gs_geo over rows [r0, r1) of one colour block.
+template <typename T, typename TR>
+void gs_geo_launch(Context* c, const Level& L, const T* val, const TR* rhs, T* x, int r0, int r1, double* dot) {
+  const GeoPhase& geo = L.geo_cols->block[sweep_at(L, r0)];
+  if constexpr (sizeof(T) == 8) {
+    if (dot) {
+      auto k = k_gs_geo<T, TR, true>;
+      const int g = std::min(grid_of(c, k, r1 - r0), kDotStride);
+      launch_early(c->stream, k, g, kThreads, 0, val, L.pitch, rhs, x, r0, r1, sink_of(L), dot, geo);
+      return;
+    }
+  }
+  auto k = k_gs_geo<T, TR, false>;
+  launch_early(c->stream, k, grid_of(c, k, r1 - r0), kThreads, 0, val, L.pitch, rhs, x, r0, r1, sink_of(L), nullptr,
+               geo);
 }
 
 template <typename T, typename TR, bool FIRST>
 void gs_dispatch(Context* c, const Level& L, int cfg, const T* val, const TR* rhs, T* x, int r0, int r1,
                  uint32_t mask, double* dot = nullptr) {
+  if constexpr (!FIRST) {
+    if (cfg == kGeoCfg && mask == kAllSlots && L.geo_cols) {
+      if (r1 > r0) gs_geo_launch<T, TR>(c, L, val, rhs, x, r0, r1, dot);
+      return;
+    }
+  }
   switch (usable_cfg(cfg, r0)) {
     case 0: gs_launch<T, TR, FIRST, 0>(c, L, val, rhs, x, r0, r1, mask, dot); break;
     case 1: gs_launch<T, TR, FIRST, 1>(c, L, val, rhs, x, r0, r1, mask, dot); break;
@@ -852,9 +875,11 @@ void pick_first(const float (&t)[kColours][kGsConfigs], int (&at)[kColours], int
 // problem's levels took 11-216 ms, and single launches of a few microseconds
 // are not told apart reliably: a step of 96^3 ran in 110 or 181 us from one
 // problem to the next). HPCG_B200_TUNE=1: time them all the same.
-//  - phases of all slots: the bulk-copy pipeline at every size (its early launch
-//    also hides a small phase's start; level 0 of 104^3: 0.44 against 0.54 ms an
-//    iteration with the tuner's pick);
+//  - phases of all slots: up to two rounds of blocks on the SMs k_gs_geo, whose
+//    threads request their rows' values before the phase before has ended (a
+//    symmetric step of 64^3: 55 against 62 us, 80^3: 66 against 84, 104^3: 120
+//    against 130); above that the bulk-copy pipeline (128^3: 193 against 213; level
+//    0 of 384^3 the more so);
 //  - first-sweep phases: k_gs_first_geo, one row a thread in FP64 (384^3: 1.36 ms a
 //    sweep, two rows 1.47, bulk copies 2.15, the tuner's register mix 1.53), two in
 //    FP32 once the phases leave the L2 (384^3: 0.81 against 0.84 ms; 128^3: 85
@@ -864,6 +889,8 @@ void pick_first(const float (&t)[kColours][kGsConfigs], int (&at)[kColours], int
 //    stream (384^3: 1.04 ms; 128^3: 43 us, in storage order 41).
 constexpr int kBeyondL2 = 4 << 20;  // rows: 32 MB a vector, 900 MB of values
 
+constexpr int kGeoRows = 2 * 2 * 148 * kThreads;  // rows of a phase: two rounds of two blocks of k_gs_geo on an SM
+
 bool by_rule(const Level& L) {
   const char* e = std::getenv("HPCG_B200_TUNE");
   return L.geo_cols && !(e && *e && e[0] != '0');
@@ -871,7 +898,7 @@ bool by_rule(const Level& L) {
 
 void rule_config(Level& L) {
   const bool large = L.n >= kBeyondL2;
-  L.gs_sched = kBulkCfg;
+  L.gs_sched = L.n / kColours <= kGeoRows ? kGeoCfg : kBulkCfg;
   L.gs_first = kGeoCfg;
   for (int s = 0; s < kColours; ++s) L.gs_first_at[s] = large && s == kColours - 1 ? kBulkCfg : kGeoCfg;
   L.mv_sched = kBulkMvCfg;
@@ -880,7 +907,7 @@ void rule_config(Level& L) {
 
 void rule_config32(Level& L) {
   const bool large = L.n >= kBeyondL2;
-  L.gs_sched32 = kBulkCfg;
+  L.gs_sched32 = L.n / kColours <= kGeoRows ? kGeoCfg : kBulkCfg;
   L.gs_first32 = large ? kGeoCfg + 1 : kGeoCfg;
   for (int s = 0; s < kColours; ++s)
     L.gs_first32_at[s] = large && s == kColours - 1 ? kBulkCfg : L.gs_first32;
