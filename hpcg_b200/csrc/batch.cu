@@ -1486,6 +1486,7 @@ int hpcg_b200_batch_cg_mixed(hpcg_b200_batch* B, const double* const* b, double*
   HB_CK(cudaSetDevice(B->device));
   Context* c = B->ctx;
   for (int p = 0; p < B->m; ++p) {
+    if (B->bulk) HB_TRY(prepare_f32(B->probs[p]));  // (a member's values may have been set since)
     HB_TRY(load_vector(B->probs[p], 0, b[p], B->probs[p]->b));
     HB_TRY(load_vector(B->probs[p], 0, x[p], B->probs[p]->x));
   }

@@ -198,7 +198,9 @@ struct Level {
   int64_t pitch = 0;         // slot stride (>= n+next+1, multiple of 256)
   double* val = nullptr;     // [27][pitch]
   int* col = nullptr;        // [27][pitch]
-  float* val32 = nullptr;    // FP32 copy for the mixed-precision V-cycle (built on first use), blocked
+  float* val32 = nullptr;    // FP32 copy for the mixed-precision V-cycle (built on first use), blocked; it keeps
+                             // its address: captured graphs and a batch's work lists hold it
+  bool old32 = false;        // val has changed since val32 was written
   int* col32 = nullptr;      // its columns in the same blocked layout (mat_index<float>)
   int* new2old = nullptr;    // [n] colour row -> natural row
   int* old2new = nullptr;    // [n]

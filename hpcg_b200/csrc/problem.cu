@@ -677,13 +677,7 @@ int hpcg_b200_set_diagonal(hpcg_b200_problem* p, const double* diagonal) {
   k_set_diag<<<grid_for(c, L.n, 256, 8), 256, 0, c->stream>>>(src, L.old2new, L.val + kDiagSlot * L.pitch, L.n);
   HB_CK(cudaGetLastError());
   if (L.valt) HB_TRY(tail_values(p, 0));
-  if (L.val32) {  // the FP32 copy is rebuilt on next use
-    dev_free(L.val32);
-    L.val32 = nullptr;
-    dev_free(L.col32);
-    L.col32 = nullptr;
-    drop_coarse_graph(p, 1);  // it holds the old copy's addresses
-  }
+  L.old32 = true;  // the FP32 copy is rewritten on next use
   HB_CK(cudaStreamSynchronize(c->stream));
   return HPCG_B200_OK;
 }
@@ -719,13 +713,7 @@ int hpcg_b200_set_values(hpcg_b200_problem* p, int level, const double* values27
     set_error("set_values", e);
     return status_of(e);
   }
-  if (L.val32) {
-    dev_free(L.val32);
-    L.val32 = nullptr;
-    dev_free(L.col32);
-    L.col32 = nullptr;
-    drop_coarse_graph(p, 1);  // it holds the old copy's addresses
-  }
+  L.old32 = true;  // the FP32 copy is rewritten on next use
   return HPCG_B200_OK;
 }
 

@@ -1378,18 +1378,22 @@ int ensure_f32(hpcg_b200_problem* P) {
   Context* c = P->ctx;
   for (int l = 0; l < P->nlev; ++l) {
     Level& L = P->lev[l];
-    if (!L.val32) {
+    if (!L.val32 || !L.col32) {
       const int64_t cnt = blocked_entries(L.pitch, kRowBlock32);
-      HB_TRY(dev_alloc((void**)&L.val32, sizeof(float) * cnt, &P->bytes));
+      if (!L.val32) HB_TRY(dev_alloc((void**)&L.val32, sizeof(float) * cnt, &P->bytes));
+      L.old32 = true;
       HB_TRY(dev_alloc((void**)&L.col32, sizeof(int) * cnt, &P->bytes));
       HB_CK(cudaMemsetAsync(L.val32, 0, sizeof(float) * cnt, c->stream));
       HB_CK(cudaMemsetAsync(L.col32, 0, sizeof(int) * cnt, c->stream));
+    }
+    if (L.old32) {
       k_block32<<<grid_for(c, (int64_t)kSlots * L.pitch, kThreads, kPerSm), kThreads, 0, c->stream>>>(
           L.val, L.col, L.pitch, L.val32, L.col32);
       HB_CK(cudaGetLastError());
       // a Gauss-Seidel phase launched next may read the copy before this
       // kernel is done (its producer does not wait): finish it here
       HB_TRY(stream_sync(c));
+      L.old32 = false;
     }
     if (!L.r32) {
       HB_TRY(dev_alloc((void**)&L.r32, sizeof(float) * L.pitch, &P->bytes));
