@@ -8,23 +8,23 @@ namespace hb {
 
 namespace {
 
-// Largest number of rows a block may have in one colour phase. 256 rows are one
-// chunk of a block's threads; each further chunk adds its own chain, while a
-// phase spread over every SM costs its launch whatever its size. Whole V-cycles
-// measured with the level in and out of this launch, FP64: 256 rows (32^3) 134
-// against 174 us, 400 rows (40x40x32) 169 against 181, 576 rows 194 against 194,
-// 800 rows (40^3) 219 against 186; FP32: 576 rows 183 against 191, 800 rows 195
-// against 189. A lone step also brings x in and its choice is between two
-// launches' worth of set-up: 256 rows 51 against 56 us, 400 rows 66 against 58.
+// Largest number of rows a block may have in one colour phase: one chunk of a
+// block's threads. Each further chunk adds its own chain, while a phase spread
+// over every SM costs its launch whatever its size. CG per iteration with the level
+// in and out of this launch, FP64: 256 rows (32^3) 136 against 139 us, 288 rows
+// (36x32x32 below 72x64x64) 218 against 194, 384 rows 218 against 194; FP32, whose
+// launched phases read half the bytes: 256 rows 137 against 133, 288 rows 202 against
+// 188. A lone step also brings x in: 64 rows (16^3) 43 against 47 us, 144 rows
+// (24^3) 49 against 47, 256 rows 51 against 47.
 // Measurement knob: HPCG_B200_TAIL_ROWS.
 int max_rows(bool f32) {
   static const int forced = [] {
     const char* e = std::getenv("HPCG_B200_TAIL_ROWS");
     return e && *e ? std::atoi(e) : 0;
   }();
-  return forced > 0 ? forced : f32 ? 640 : 448;
+  return forced > 0 ? forced : f32 ? 240 : 256;
 }
-constexpr int kStepRows = 288;
+constexpr int kStepRows = 96;
 constexpr int kMaxSmem = 200 * 1024;
 // A level with at most this many rows to a colour stays on one block: its
 // phases then end at the block's own barrier instead of the cluster's.
