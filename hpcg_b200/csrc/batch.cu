@@ -5,10 +5,12 @@
 // Every step of an iteration is ONE kernel launch for the whole batch: the
 // launch walks a work list of row tiles that spans all problems (a colour phase
 // of every problem's level, a restriction, a vector update...), so a batch of
-// small problems costs the launches of one. The iteration loop itself is one
+// small problems costs the launches of one (and, in the form chosen by default,
+// the small levels of all problems are one launch). The iteration loop itself is one
 // CUDA graph launch: a conditional while node repeats the iteration while any
 // problem is still above its tolerance and the iteration limit is not reached;
-// problems that have converged skip their tiles. No kernel waits on another.
+// problems that have converged skip their tiles. No kernel waits on another (an
+// early launch waits on the device for the kernel before it).
 #include <cmath>
 #include <cstdlib>
 #include <cstring>

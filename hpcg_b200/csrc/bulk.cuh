@@ -26,8 +26,8 @@ namespace hb {
 // group and no wait on a barrier can start more than one phase early (an
 // mbarrier parity wait cannot tell phase n from phase n - 2). The kernels that
 // use it keep the slot order of their register-pipelined twins: the same bits.
-// A first sweep copies all slots too (it reads about half), so the autotuner
-// usually keeps another configuration for it.
+// A first sweep copies all slots too (it reads about half), so it usually runs
+// another configuration.
 // Every wait gives up after kBulkWaitNs of global time: the thread then sets
 // the context's fault word (host-mapped; stream_sync turns it into
 // HPCG_B200_ERR_TIMEOUT) and stops; before its block exits the producer waits,
@@ -83,10 +83,9 @@ static_assert(pack_rec(1) % 16 == 0 && pack_rec(2) % 16 == 0 && pack_rec(kPackDi
 
 // Shape of a pipeline: G consumer groups of kBulkRows x LANES threads, each
 // with a ring of RING stages of one tile. A stage holds the tile's values and
-// its columns: 32-bit (PW = 0), or the packed record of form PW (1, 2: offsets
-// of PW bytes; 3: diagonal), or, with PW = -1, a record whose form each tile
-// states (the batched kernel, whose tiles come from several levels): staged
-// for the largest one, each fill expecting its own record's bytes. Stages are rounded up to
+// its columns: 32-bit (PW = 0), the packed record of form PW (1, 2: offsets
+// of PW bytes; 3: diagonal), or none (kPackGeo: the values alone, the columns from
+// the grid). Stages are rounded up to
 // 128 bytes (tensor copies land on 128-byte boundaries): FP64 stages are 41.5
 // KB with 32-bit columns (33.9 / 30.5 / 28.3 KB with 16-bit offsets, 8-bit
 // offsets, the diagonal form) and FP32 one-block stages 27 KB (20.4 / 17 /
@@ -114,19 +113,19 @@ struct BulkShape {
   static constexpr int threads = 32 + groups * group_threads;  // producer warp + consumers
   static constexpr int block_value_bytes = kSlots * kBulkRows * (int)sizeof(T);
   static constexpr int block_col_bytes =
-      geo ? 0 : PW == 0 ? kSlots * kBulkRows * (int)sizeof(int) : pack_rec(PW < 0 ? 2 : PW);
+      geo ? 0 : PW == 0 ? kSlots * kBulkRows * (int)sizeof(int) : pack_rec(PW);
   static constexpr int value_bytes = block_value_bytes * TB;
   static constexpr int col_bytes = block_col_bytes * TB;
-  static_assert(TB == 1 || (TB == 2 && bulk_whole_tile<T>() && PW >= 0 && LANES == 1),
-                "tiles of two blocks: whole-tile copies, one record form, one thread per row");
-  static constexpr int tx_bytes = value_bytes + col_bytes;  // bytes landing in a stage per fill (PW >= 0)
+  static_assert(TB == 1 || (TB == 2 && bulk_whole_tile<T>() && LANES == 1),
+                "tiles of two blocks: whole-tile copies, one thread per row");
+  static constexpr int tx_bytes = value_bytes + col_bytes;  // bytes landing in a stage per fill
   static constexpr int stage_bytes = (tx_bytes + 127) / 128 * 128;
   // stages + per stage two barriers and the tile's first row + slack to align
   // the stages to 128 bytes (tensor copies)
   static constexpr int smem = stages * stage_bytes + 3 * stages * (int)sizeof(uint64_t) + 128;
   static_assert(smem <= 227 * 1024, "shared memory of one block");
   static_assert(threads <= 1024, "threads of one block");
-  static_assert(PW >= -1 && PW <= kPackGeo, "column form");
+  static_assert(PW >= 0 && PW <= kPackGeo, "column form");
 };
 // The shapes in use: rings of two stages (measured at 512^3: two groups of two
 // stages beat four groups of one for the Gauss-Seidel phases by 8% and tied for
@@ -167,7 +166,7 @@ struct BulkShape {
 #define HB_GS32_TILE 2
 #endif
 // Whether the Gauss-Seidel phases, the SpMV and the restriction hand a stage
-// back once the row's values and columns are in registers (bulk_tiles_src's
+// back once the row's values and columns are in registers (bulk_tiles'
 // EARLY), per value type. Measured at 512^3 on one box: the FP32 phases went
 // from 10.01 to 9.09 ms per iteration; the FP64 phases (15.68 -> 15.85 ms),
 // the SpMV (5.60 -> 5.59 ms) and the FP64 restriction (0.73 -> 0.76 ms) did
@@ -215,17 +214,16 @@ template <typename T>
 __host__ __device__ constexpr int gs_ring() {
   return sizeof(T) == 8 ? HB_BULK_RING : HB_GS32_RING;
 }
-// blocks per tile of the Gauss-Seidel phases: FP32 with one record form (the
-// batched kernel's per-tile forms keep one block)
-template <typename T, int PW>
+// blocks per tile of the Gauss-Seidel phases
+template <typename T>
 __host__ __device__ constexpr int gs_blocks() {
-  return sizeof(T) == 4 && PW >= 0 ? HB_GS32_TILE : 1;
+  return sizeof(T) == 4 ? HB_GS32_TILE : 1;
 }
 template <typename T, int PW = 0>
 using GsShape = BulkShape<T,
-                          fit_groups<T, PW, gs_blocks<T, PW>()>(sizeof(T) == 8 ? HB_GS64_GROUPS : HB_GS32_GROUPS,
+                          fit_groups<T, PW, gs_blocks<T>()>(sizeof(T) == 8 ? HB_GS64_GROUPS : HB_GS32_GROUPS,
                                                                 gs_ring<T>()),
-                          gs_ring<T>(), 1, PW, gs_blocks<T, PW>()>;
+                          gs_ring<T>(), 1, PW, gs_blocks<T>()>;
 template <typename T, int PW = 0>
 using SpmvShape = BulkShape<T, fit_groups<T, PW>(sizeof(T) == 8 ? HB_SPMV_GROUPS : HB_SPMV32_GROUPS, sizeof(T) == 8 ? HB_SPMV_RING : HB_BULK_RING),
                             sizeof(T) == 8 ? HB_SPMV_RING : HB_BULK_RING, 1, PW>;
@@ -261,14 +259,11 @@ __device__ __forceinline__ int stage_col(const int* sc, int k, int t, int sink) 
     return o == pack_sink(2) ? sink : sc[k] + (int)o;
   } else if constexpr (PW == kPackGeo) {
     return 0;  // not from the stage: GeoRow::col
-  } else if constexpr (PW == kPackDiag) {
+  } else {
+    static_assert(PW == kPackDiag, "column form");
     // the warp's 32 rows share one word of sink bits (a broadcast load)
     const unsigned bits = reinterpret_cast<const unsigned*>(sc + kPackBaseWords)[k * (kBulkRows / 32) + (t >> 5)];
     return (bits >> (t & 31)) & 1u ? sink : sc[k] + t;
-  } else {
-    const int w = sc[kSlots];
-    return w == 1 ? stage_col<1>(sc, k, t, sink) : w == 2 ? stage_col<2>(sc, k, t, sink)
-                                                           : stage_col<kPackDiag>(sc, k, t, sink);
   }
 }
 
@@ -359,38 +354,48 @@ __device__ __forceinline__ void record_fault(unsigned* fault, unsigned code) {
 
 // Where a tile comes from: its first row and, when the tile is one block of
 // the layout (whole-tile copies), the addresses of its value and column blocks;
-// with packed columns, the address of its record and (read only when the
-// shape's offset width is per tile, PW = -1) the record's bytes.
+// with packed columns, the address of its record.
 template <typename T>
 struct TileSrc {
   int64_t q0;
   const T* vals;
   const int* cols;
   const unsigned char* rec;
-  int rec_bytes;
   const CUtensorMap* map = nullptr;  // FP64 tiles of bulk_tiles_driven: the matrix the tile is of
 };
 
 // The producer/consumer pipeline of the bulk-copy kernels, run by the whole
-// block. The block's tiles are blockIdx.x, + gridDim.x, ... below ntiles, less
-// those for which skip(tile) holds (every thread of the block must get the same
-// answer); the i-th tile kept goes to consumer group i mod G. src(tile) gives
-// the tile's TileSrc; the tensor maps (FP64 tiles only) are kernel parameters.
-// Each consumer thread calls row(tile, q0, sv, sc, t) for
+// block, over one matrix (val, col or the packed records colp, pitch). The
+// block's tiles are blockIdx.x, + gridDim.x, ... below ntiles, tile `tile`
+// starting at row first_row(tile) (a multiple of kBulkRows with packed columns or
+// whole-tile copies); its i-th goes to consumer group i mod G. The tensor maps
+// (FP64 tiles only) are kernel parameters.
+// Each consumer thread calls row(q0, sv, sc, t) for
 // every tile of its group, t its index in the group (row t / LANES of the tile,
 // lane t % LANES), with the tile's values sv[k * kBulkRows + row] and columns
 // on chip: sc[k * kBulkRows + row], or the packed record at sc
 // (stage_col<Shape::pack> reads any of them). The tile's first row q0 comes
-// from the producer through the stage (it computed src(tile) for the copies),
+// from the producer through the stage (it computed it for the copies),
 // so the consumers' loads wait on no index arithmetic of their own.
-// EARLY: row(tile, q0, sv, sc, t, release) takes what it needs of the stage
+// EARLY: row(q0, sv, sc, t, release) takes what it needs of the stage
 // into registers and calls release() (exactly once, on every path) to hand
 // the stage back to the producer before it gathers and computes, so a stage
 // is held for its shared-memory reads only and the ring keeps more fills in
 // flight; otherwise the stage is released after row() returns.
-template <typename T, typename Shape, bool EARLY = false, typename Src, typename Skip, typename RowFn>
-__device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, RowFn row, unsigned* fault,
-                                               const CUtensorMap* tm_val, const CUtensorMap* tm_col) {
+template <typename T, typename Shape, bool EARLY = false, typename FirstRow, typename RowFn>
+__device__ __forceinline__ void bulk_tiles(const T* __restrict__ val, const int* __restrict__ col, int64_t pitch,
+                                           int ntiles, FirstRow first_row, RowFn row, unsigned* fault,
+                                           const CUtensorMap& tm_val, const CUtensorMap& tm_col,
+                                           const unsigned char* colp = nullptr) {
+  auto src = [&](int tile) {
+    const int64_t q0 = first_row(tile);
+    TileSrc<T> ts{};
+    ts.q0 = q0;
+    ts.vals = val + mat_index<T>(0, q0, pitch);
+    ts.cols = col + mat_index<T>(0, q0, pitch);
+    if constexpr (Shape::packed) ts.rec = colp + (q0 / kBulkRows) * pack_rec(Shape::pack);
+    return ts;
+  };
   constexpr int G = Shape::groups;
   constexpr int RING = Shape::ring;
   constexpr int S = Shape::stages;
@@ -412,9 +417,7 @@ __device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, R
   __syncthreads();
   // Under a programmatic dependent launch the producer streams the first tiles
   // while the previous kernel finishes: it reads only the matrix, and every
-  // kernel that writes a matrix array is followed by a stream synchronisation.
-  // (The batched kernel's skip predicate reads convergence flags; it is
-  // launched without the attribute, so the wait is already over.) The
+  // kernel that writes a matrix array is followed by a stream synchronisation. The
   // consumers read and write the vectors: they wait for that kernel first.
   if (threadIdx.x == 0) griddep_launch_dependents();
   const int warp = threadIdx.x >> 5;
@@ -426,13 +429,11 @@ __device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, R
     int last[S];  // last fill issued into each stage (-1: none)
 #pragma unroll
     for (int s = 0; s < S; ++s) last[s] = -1;
-    int i = 0;  // tiles kept so far: tile i goes to group i % G, as its (i / G)-th
+    int i = 0;  // tiles so far: tile i goes to group i % G, as its (i / G)-th
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-      if (skip(tile)) continue;
       const int kg = i / G;
       const int s = (i % G) * RING + kg % RING, use = kg / RING;
       const TileSrc<T> ts = src(tile);
-      const int rec_bytes = Shape::pack < 0 ? ts.rec_bytes : Shape::col_bytes;
       int ok = 1;
       if (lane == 0) {
         if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1)) {
@@ -440,7 +441,7 @@ __device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, R
           ok = 0;
         } else {
           first[s] = ts.q0;  // released to the consumers by the arrival below
-          mbar_expect_tx(&full[s], Shape::value_bytes + rec_bytes);
+          mbar_expect_tx(&full[s], Shape::tx_bytes);
         }
       }
       if (!__shfl_sync(0xffffffffu, ok, 0)) break;
@@ -451,16 +452,16 @@ __device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, R
         if (lane == 0) bulk_g2s(sv, ts.vals, VB, &full[s], policy);
       } else {
         // rows q0 .. q0 + kBulkRows of all 27 slots, [slot][row] in shared memory
-        if (lane == 0) tma_load_2d(sv, tm_val, (int)ts.q0, 0, &full[s], policy);
+        if (lane == 0) tma_load_2d(sv, &tm_val, (int)ts.q0, 0, &full[s], policy);
       }
       if constexpr (Shape::geo) {
         // no columns to fetch
       } else if constexpr (Shape::packed) {
-        if (lane == 1) bulk_g2s(sc, ts.rec, rec_bytes, &full[s], policy);
+        if (lane == 1) bulk_g2s(sc, ts.rec, Shape::col_bytes, &full[s], policy);
       } else if constexpr (bulk_whole_tile<T>()) {
         if (lane == 1) bulk_g2s(sc, ts.cols, Shape::col_bytes, &full[s], policy);
       } else {
-        if (lane == 1) tma_load_2d(sc, tm_col, (int)ts.q0, 0, &full[s], policy);
+        if (lane == 1) tma_load_2d(sc, &tm_col, (int)ts.q0, 0, &full[s], policy);
       }
 #pragma unroll
       for (int u = 0; u < S; ++u)
@@ -479,9 +480,8 @@ __device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, R
     griddep_wait();
     const int g = (warp - 1) / (Shape::group_threads / 32);   // consumer group
     const int t = (threadIdx.x - 32) % Shape::group_threads;  // index in the group
-    int i = 0;                                                // tiles kept so far
+    int i = 0;                                                // tiles so far
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-      if (skip(tile)) continue;
       if (i % G == g) {
         const int kg = i / G;
         const int s = g * RING + kg % RING, use = kg / RING;
@@ -496,9 +496,9 @@ __device__ __forceinline__ void bulk_tiles_src(int ntiles, Src src, Skip skip, R
         const int* sc = reinterpret_cast<const int*>(smem + s * SB + VB + h * Shape::block_col_bytes);
         const int tb = t - h * Shape::block_threads;
         if constexpr (EARLY) {
-          row(tile, q0, sv, sc, tb, [&] { mbar_arrive(&empty[s]); });
+          row(q0, sv, sc, tb, [&] { mbar_arrive(&empty[s]); });
         } else {
-          row(tile, q0, sv, sc, tb);
+          row(q0, sv, sc, tb);
           mbar_arrive(&empty[s]);
         }
       }
@@ -601,29 +601,6 @@ __device__ __forceinline__ void bulk_tiles_driven(int ntiles, Src src, Skip skip
           t, [&] { mbar_arrive(&empty[s]); });
     }
   }
-}
-
-// The common case: one matrix (val, col or the packed records colp, pitch),
-// tile `tile` starting at row first_row(tile) (a multiple of kBulkRows with
-// packed columns or whole-tile copies), no tile skipped; row(q0, sv, sc, t).
-// EARLY: row(q0, sv, sc, t, release), as bulk_tiles_src's.
-template <typename T, typename Shape, bool EARLY = false, typename FirstRow, typename RowFn>
-__device__ __forceinline__ void bulk_tiles(const T* __restrict__ val, const int* __restrict__ col, int64_t pitch,
-                                           int ntiles, FirstRow first_row, RowFn row, unsigned* fault,
-                                           const CUtensorMap& tm_val, const CUtensorMap& tm_col,
-                                           const unsigned char* colp = nullptr) {
-  bulk_tiles_src<T, Shape, EARLY>(
-      ntiles,
-      [&](int tile) {
-        const int64_t q0 = first_row(tile);
-        static_assert(Shape::pack >= 0, "one offset width per level");
-        return TileSrc<T>{q0, val + mat_index<T>(0, q0, pitch), col + mat_index<T>(0, q0, pitch),
-                          Shape::packed ? colp + (q0 / kBulkRows) * pack_rec(Shape::pack) : nullptr,
-                          Shape::col_bytes};
-      },
-      [](int) { return false; },
-      [&](int, int64_t q0, const T* sv, const int* sc, int t, auto&&... release) { row(q0, sv, sc, t, release...); },
-      fault, &tm_val, &tm_col);
 }
 
 }  // namespace hb

@@ -212,7 +212,7 @@ struct Level {
   double* x = nullptr;       // coarse solution (levels > 0), [pitch]
   float* r32 = nullptr;      // FP32 V-cycle vectors, [pitch]
   float* x32 = nullptr;
-  // kernel configuration of this level's row kernels, chosen by the autotuner
+  // kernel configuration of this level's row kernels, by rule or by timing (solver.cu)
   int gs_sched = 1;          // kernel configuration of the Gauss-Seidel phases (FP64)
   int gs_sched32 = 1;        // kernel configuration of the Gauss-Seidel phases (FP32 V-cycle)
   int gs_first32 = 1;        // ... of its first-sweep phases

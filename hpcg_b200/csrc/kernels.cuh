@@ -23,7 +23,7 @@ namespace hb {
 // (neighbours not yet swept, and the diagonal) multiply a zero and are skipped,
 // which leaves every sum bitwise unchanged.
 // ---------------------------------------------------------------------------
-// Kernel configurations the autotuner chooses from. Every configuration
+// Kernel configurations, chosen by rule or by timing (solver.cu). Every configuration
 // computes the same bits; they differ in how the loads are issued:
 //  - schedule: kPlain issues loads as the compiler schedules the slot loop;
 //    kStaged issues all masked value/column loads first (27 independent loads in
@@ -938,14 +938,6 @@ __global__ void __launch_bounds__(kThreads) k_spmv_nat(const double* __restrict_
     sum += a[k] * xv;
   }
   y[i] = sum;
-}
-
-// dst[i] = src[idx[i]]
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_gather(T* __restrict__ dst, const T* __restrict__ src,
-                                                     const int* __restrict__ idx, int n) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = src[idx[i]];
 }
 
 // w = alpha x + beta y (ComputeWAXPBY_ref.cpp:52-67; its alpha == 1 and

@@ -768,7 +768,9 @@ bool rtz_fused(const hpcg_b200_problem* P) {
   return !(L.gs_sched == kBulkCfg && L.colp && L.pack != kPackDiag && !L.geo_cols);
 }
 
-// Autotuner: per level, times each kernel configuration (load schedule x
+// Autotuner, for levels that read stored columns (and, with HPCG_B200_TUNE=1,
+// for those whose configurations follow from rule_config): times each kernel
+// configuration (load schedule x
 // registers per thread) of the Gauss-Seidel phase and of the SpMV on scratch
 // vectors (Ap as x, zprev as right-hand side on level 0; the coarse r/x pair
 // otherwise) and keeps the fastest. Every configuration computes the same bits,

@@ -185,10 +185,10 @@ int hpcg_b200_batch_problem(hpcg_b200_batch* batch, int i, hpcg_b200_problem** o
 int hpcg_b200_batch_cg_mixed(hpcg_b200_batch* batch, const double* const* b, double* const* x, int max_iter,
                              double tolerance, int* niters, double* normr, double* normr0);
 int hpcg_b200_batch_free(hpcg_b200_batch* batch);
-/* How the batch runs an iteration, chosen by timing at creation (or by
- * HPCG_B200_BATCH_PERSIST / HPCG_B200_BATCH_BULK): 0 one launch per step with
- * the colour phases on the register kernel, 1 the same on the bulk-copy
- * kernel, 2 the whole iteration as one cooperative launch whose steps are
+/* How the batch runs an iteration: 1 one launch per step on the bulk-copy
+ * kernels, the columns taken from the grids and the small levels of all problems
+ * in one launch (the default), 0 one launch per step on the register kernels
+ * (HPCG_B200_BATCH_BULK=0), 2 (HPCG_B200_BATCH_PERSIST=1) the whole iteration as one cooperative launch whose steps are
  * separated by grid barriers with bounded waits (a wait that gives up ends the
  * solve with HPCG_B200_ERR_TIMEOUT). */
 int hpcg_b200_batch_form(const hpcg_b200_batch* batch, int* form);
@@ -310,16 +310,19 @@ int hpcg_b200_level_packed(const hpcg_b200_problem* p, int level, int64_t* bytes
 int hpcg_b200_export_level(const hpcg_b200_problem* p, int level, int* new2old, int* cols, double* vals,
                            int* f2c);
 
-/* The autotuner's choices for one level (7 ints): kernel configuration of the
+/* The choices for one level (7 ints): kernel configuration of the
  * Gauss-Seidel phases, of the first-sweep phases, of the FP32 phases, of the
  * SpMV/restriction, the SpMV row order (0 storage, 1 natural, 2 slab), whether
- * the level has been tuned yet (tuning happens on first use), and the
- * configuration of the FP32 first-sweep phases. */
+ * the choice has been made yet (it is on first use), and the configuration of
+ * the FP32 first-sweep phases. A level whose columns follow from its grid takes
+ * them by rule on its size; the others, and every level with HPCG_B200_TUNE=1,
+ * time the configurations. Levels that run inside the one-launch small end of
+ * the V-cycle report theirs too, without using them there. */
 int hpcg_b200_level_config(const hpcg_b200_problem* p, int level, int* config);
 
 /* The configuration of the first forward sweep's phase at each of the 8 sweep
  * positions of one level (a phase reads 0 to 26 slots by its position, so the
- * tuner chooses per position): fp64 for the FP64 V-cycle, fp32 for the FP32
+ * choice is made per position): fp64 for the FP64 V-cycle, fp32 for the FP32
  * one (8 ints each, either may be NULL). */
 int hpcg_b200_level_first_config(const hpcg_b200_problem* p, int level, int* fp64, int* fp32);
 
