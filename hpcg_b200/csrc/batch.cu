@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(BatchShape::threads, 1)
         else
           work(items[item0 + at]);
       },
-      fault);
+      fault, false);  // (sides are multiples of 16: colours start on whole sectors)
 }
 
 // A first-sweep phase (k_gs_first_geo's arithmetic), 256 rows a tile.
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(BatchSpmv::threads, 1)
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
         if ((threadIdx.x & 31) == 0) partials[4 * (tile0[p] + q0 / kBulkRows) + row / 32] = acc;
       },
-      fault);
+      fault, true);
 }
 
 // rc = (rf - A xf) at the injected rows (ComputeMG_ref.cpp:49-51, sorted pairs)

@@ -331,20 +331,35 @@ __device__ __forceinline__ uint64_t evict_first_policy() {
 }
 // Programmatic dependent launch: a kernel launched with programmatic stream
 // serialization may start while the kernel before it on the stream finishes;
-// griddep_wait() returns once that kernel has completed and its writes are
-// visible (at once for a kernel launched without the attribute), and
-// griddep_launch_dependents() lets the next such kernel start.
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+// griddep_wait() returns once that kernel has completed and its writes are in the
+// L2 (at once for a kernel launched without the attribute), and then lets the next
+// such kernel start. Not sooner: a block's L1 is cleared when the block starts, not
+// by the wait, so a block that started while the kernel two before it still ran may
+// find lines in its SM's L1 that were read before the kernel in between rewrote
+// them (seen as residuals that differed from run to run). With the release after
+// the wait only the kernel directly before can have put lines there, and stale
+// ones are lines that it read and that another SM wrote meanwhile. `fence` drops
+// those too (0.2 us); a kernel may leave it out where no 32 bytes are read and
+// written by two blocks of the kernel before it.
+__device__ __forceinline__ void griddep_wait(bool fence = true) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (fence) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+}
 
 // The wait, and the pointers to what the kernels before may have written made new
 // to the compiler: loads through a const __restrict__ pointer or __ldg are free to
 // move across any barrier, so a kernel that was launched early must not hold the
 // address before the wait.
 template <typename... P>
+__device__ __forceinline__ void griddep_reload(P&... p) {
+  ((void)([&] { asm volatile("" : "+l"(p)::"memory"); }()), ...);
+}
+
+template <typename... P>
 __device__ __forceinline__ void griddep_wait_for(P&... p) {
   griddep_wait();
-  ((void)([&] { asm volatile("" : "+l"(p)::"memory"); }()), ...);
+  griddep_reload(p...);
 }
 
 __device__ __forceinline__ void record_fault(unsigned* fault, unsigned code) {
@@ -386,7 +401,7 @@ template <typename T, typename Shape, bool EARLY = false, typename FirstRow, typ
 __device__ __forceinline__ void bulk_tiles(const T* __restrict__ val, const int* __restrict__ col, int64_t pitch,
                                            int ntiles, FirstRow first_row, RowFn row, unsigned* fault,
                                            const CUtensorMap& tm_val, const CUtensorMap& tm_col,
-                                           const unsigned char* colp = nullptr) {
+                                           const unsigned char* colp = nullptr, bool fence = true) {
   auto src = [&](int tile) {
     const int64_t q0 = first_row(tile);
     TileSrc<T> ts{};
@@ -419,7 +434,6 @@ __device__ __forceinline__ void bulk_tiles(const T* __restrict__ val, const int*
   // while the previous kernel finishes: it reads only the matrix, and every
   // kernel that writes a matrix array is followed by a stream synchronisation. The
   // consumers read and write the vectors: they wait for that kernel first.
-  if (threadIdx.x == 0) griddep_launch_dependents();
   const int warp = threadIdx.x >> 5;
   if (warp == 0) {
     // the producer warp: lane 0 waits for a free stage and posts the byte
@@ -477,7 +491,7 @@ __device__ __forceinline__ void bulk_tiles(const T* __restrict__ val, const int*
     }
     __syncwarp();
   } else {
-    griddep_wait();
+    griddep_wait(fence);
     const int g = (warp - 1) / (Shape::group_threads / 32);   // consumer group
     const int t = (threadIdx.x - 32) % Shape::group_threads;  // index in the group
     int i = 0;                                                // tiles so far
@@ -514,7 +528,8 @@ __device__ __forceinline__ void bulk_tiles(const T* __restrict__ val, const int*
 // neither the list nor what decides the skipping. Columns from the grid (values
 // only), early release: row(tag, sv, t, release), t the row in the tile.
 template <typename T, typename Shape, typename Src, typename Skip, typename RowFn>
-__device__ __forceinline__ void bulk_tiles_driven(int ntiles, Src src, Skip skip, RowFn row, unsigned* fault) {
+__device__ __forceinline__ void bulk_tiles_driven(int ntiles, Src src, Skip skip, RowFn row, unsigned* fault,
+                                                  bool fence) {
   constexpr int G = Shape::groups;
   constexpr int RING = Shape::ring;
   constexpr int S = Shape::stages;
@@ -533,7 +548,6 @@ __device__ __forceinline__ void bulk_tiles_driven(int ntiles, Src src, Skip skip
     mbar_init_fence();
   }
   __syncthreads();
-  if (threadIdx.x == 0) griddep_launch_dependents();
   const int warp = threadIdx.x >> 5;
   if (warp == 0) {
     if (threadIdx.x == 0) {
@@ -585,7 +599,7 @@ __device__ __forceinline__ void bulk_tiles_driven(int ntiles, Src src, Skip skip
     }
     __syncwarp();
   } else {
-    griddep_wait();
+    griddep_wait(fence);
     const int g = (warp - 1) / (Shape::group_threads / 32);
     const int t = (threadIdx.x - 32) % Shape::group_threads;
     for (int kg = 0;; ++kg) {

@@ -323,7 +323,6 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) * R * __builtin_popcount(M
                    int sink, const __grid_constant__ GeoPhase geo) {
   const int tile = kThreads * R;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  griddep_launch_dependents();
   bool waited = false;
   for (int b0 = r0 + blockIdx.x * tile; b0 < r1; b0 += gridDim.x * tile) {
     const int q0 = b0 + warp * 32 * R + lane;
@@ -339,7 +338,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) * R * __builtin_popcount(M
       }
     }
     if (!waited) {  // the first rows' values are on their way while the phase before drains
-      griddep_wait_for(rhs, x);
+      griddep_wait(geo.shared);
+      griddep_reload(rhs, x);
       waited = true;
     }
 #pragma unroll
@@ -379,7 +379,6 @@ template <typename T, typename TR, bool DOT>
 __global__ void __launch_bounds__(kThreads, 2)
     k_gs_geo(const T* __restrict__ val, int64_t pitch, const TR* __restrict__ rhs, T* x, int r0, int r1, int sink,
              double* __restrict__ dot, const __grid_constant__ GeoPhase geo) {
-  griddep_launch_dependents();
   bool waited = false;
   double acc = 0.0;
   for (int b0 = r0 + blockIdx.x * kThreads; b0 < r1; b0 += gridDim.x * kThreads) {
@@ -390,7 +389,8 @@ __global__ void __launch_bounds__(kThreads, 2)
       for (int k = 0; k < kSlots; ++k) a[k] = __ldg(val + mat_index<T>(k, q, pitch));
     }
     if (!waited) {
-      griddep_wait_for(rhs, x);
+      griddep_wait(geo.shared);
+      griddep_reload(rhs, x);
       waited = true;
     }
     if (q < r1) {
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(GsShape<T, PW>::threads, 1)
           if (DOT) acc += (double)rhs[q] * (double)out;
         }
       },
-      fault, tm_val, tm_col, colp);
+      fault, tm_val, tm_col, colp, PW != kPackGeo || geo.shared);
   if (DOT) {
     const double s = block_sum(acc);
     if (threadIdx.x == 0) dot[blockIdx.x] = s;
@@ -850,10 +850,12 @@ __global__ void __launch_bounds__(RestrictShape<T, PW>::threads, 1)
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_prolong(const int* __restrict__ tf, const int* __restrict__ tq,
                                                       const T* __restrict__ xc, T* __restrict__ xf, int nc) {
-  griddep_launch_dependents();
   griddep_wait_for(xc, xf);
   const int stride = gridDim.x * blockDim.x;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nc; t += stride) xf[tf[t]] += xc[tq[t]];
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nc; t += stride) {
+    T* at = xf + tf[t];
+    *at = __ldcg(at) + xc[tq[t]];  // (past the L1: neighbours in the 32 bytes may be another block's)
+  }
 }
 
 // ---- vectors ----------------------------------------------------------------
@@ -965,7 +967,6 @@ __global__ void __launch_bounds__(kThreads) k_waxpby(int n, double alpha, const 
 template <bool TWO>
 __global__ void __launch_bounds__(kThreads) k_dot(int n, const double* __restrict__ x, const double* __restrict__ y,
                                                   const double* __restrict__ y2, double* __restrict__ partials) {
-  griddep_launch_dependents();
   griddep_wait_for(x, y, y2);
   const int stride = gridDim.x * blockDim.x;
   double acc = 0.0, acc2 = 0.0;
@@ -1035,7 +1036,6 @@ __global__ void __launch_bounds__(kThreads) k_widen_dot(int n, const float* __re
                                                         const double* __restrict__ r, double* __restrict__ z,
                                                         const double* __restrict__ zprev,
                                                         double* __restrict__ partials) {
-  griddep_launch_dependents();
   griddep_wait_for(x32, r, z, zprev);
   const int stride = gridDim.x * blockDim.x;
   double acc = 0.0, acc2 = 0.0;
@@ -1085,7 +1085,6 @@ __device__ __forceinline__ void apply_fin(int op, double sum, double sum2, Scala
 // at partials[nparts..] for kFinFlex), then the scalar update of `op`.
 __global__ void __launch_bounds__(kThreads) k_finalize(const double* __restrict__ partials, int nparts, int op,
                                                        Scalars* s, double* out) {
-  griddep_launch_dependents();
   griddep_wait_for(partials, s, out);
   double acc = 0.0, acc2 = 0.0;
   if (op == kFinMax) {
@@ -1109,7 +1108,6 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const double* __restrict_
 constexpr int kWideParts = kColours * kDotStride, kWideThreads = 1024;
 __global__ void __launch_bounds__(kWideThreads) k_finalize_wide(const double* __restrict__ partials, int op,
                                                                 Scalars* s, double* out) {
-  griddep_launch_dependents();
   griddep_wait_for(partials, s, out);
   static_assert(kWideParts == 16 * kWideThreads, "eight pairs a thread");
   const double2* p = reinterpret_cast<const double2*>(partials) + threadIdx.x;
@@ -1141,7 +1139,6 @@ __global__ void k_finalize_ranks(const double* __restrict__ vals, int nvals, int
 // first (iteration 1): p = z (CG.cpp:109), x untouched.
 __device__ __forceinline__ void update_px(int n, const double* __restrict__ z, double* p, double* x,
                                           const Scalars* __restrict__ s, bool first) {
-  griddep_launch_dependents();
   griddep_wait_for(z, p, x, s);
   const double beta = s->beta, alpha = s->alpha;
   const int stride = gridDim.x * blockDim.x;
@@ -1171,7 +1168,6 @@ __global__ void __launch_bounds__(kThreads) k_update_px_iter(int n, const double
 __global__ void __launch_bounds__(kThreads) k_update_r(int n, double* r, const double* __restrict__ Ap,
                                                        const Scalars* __restrict__ s, double* __restrict__ partials,
                                                        float* __restrict__ r32 = nullptr) {
-  griddep_launch_dependents();
   griddep_wait_for(r, Ap, s);
   const double malpha = -s->alpha;
   const int stride = gridDim.x * blockDim.x;

@@ -356,7 +356,6 @@ __device__ __forceinline__ void tail_run(const TailDesc<T>& D, const T* __restri
   TailRow* table = reinterpret_cast<TailRow*>(smem + D.elems);
   const int rank = (int)cluster_rank();
   TailWait wait{&sync, fault, 0, 0u, false};
-  griddep_launch_dependents();
   if (threadIdx.x == 0) {
     mbar_init(&sync.bar[0], 1);
     mbar_init(&sync.bar[1], 1);
