@@ -37,7 +37,14 @@ METRIC = "HPCG GFLOP/s & HBM GB/s at 512^3; FP32-MG vs FP64 time to 1e-9 residua
 # a level's column index as the kernels read it (hpcg_b200_level_packed): the
 # "column_form" fields of the JSON line hold these codes
 COLUMN_FORMS = {0: "32-bit columns", 1: "8-bit offsets", 2: "16-bit offsets",
-                3: "diagonal form: 27 bases and 27 x 128 sink bits per 128-row tile"}
+                3: "diagonal form: 27 bases and 27 x 128 sink bits per 128-row tile",
+                4: "columns taken from the grid"}
+
+
+def column_form(P, level):
+    """The column form a level's kernels read: a generated problem on one rank
+    takes its columns from the grid unless a stored form is asked for."""
+    return P.level_pack_width(level) if os.environ.get("HPCG_B200_PACKED") else 4
 
 
 def parse():
@@ -121,7 +128,7 @@ def profile_case(n):
     P.CG_mixed(b, x, 3, 0.0)
     torch.cuda.synchronize()
     print(json.dumps({"case": n, "configs": [P.level_config(l) for l in range(4)],
-                      "column_forms": [P.level_pack_width(l) for l in range(4)],
+                      "column_forms": [column_form(P, l) for l in range(4)],
                       "level_config": P.level_config_string()}))
     P.free()
     return 0
@@ -446,7 +453,7 @@ def mixed_vs_fp64(P, b, lib_stream, tol, max_iter=2000, profile_iters=20):
     fi_ms, fi_l, fi_rows = B.profile_read(B.PROF_GS32_FIRST, dev)
     B.profile(False, dev)
     peak, _ = measured_peak_hbm()
-    pack = P.level_pack_width(0) if P.level_config(0)["gs32"] == 10 else 0
+    pack = column_form(P, 0) if P.level_config(0)["gs32"] in (10, 11) else 0
     full_gbs = metrics.gs_phase_bytes(fu_rows, n, vb=4, pack=pack) / (fu_ms * 1e-3) / 1e9 if fu_ms else None
     first_gbs = metrics.first_sweep_bytes(fi_rows, vb=4) / (fi_ms * 1e-3) / 1e9 if fi_ms else None
     return {"fp64": {"iters": it64, "seconds": round(t64, 3), "scaled_residual": nr64 / nr064},
@@ -578,9 +585,9 @@ def b200_arm(args, rank, world, local_rank):
     flops_step = metrics.hpcg_flops(n, n, n, args.iters)
     value = flops_step * args.steps * world / (ms * 1e-3) / 1e9
     # the iteration's algorithmic bytes as the library's kernels move them,
-    # with each level's column index as stored (8-bit or 16-bit offsets, or
-    # 32-bit columns)
-    packs = tuple(P.level_pack_width(l) for l in range(4))
+    # with each level's column index as read (none where the columns come from
+    # the grid; else 8-bit or 16-bit offsets, or 32-bit columns)
+    packs = tuple(column_form(P, l) for l in range(4))
     # r'z rides on the post-smoother except on 8-bit / 16-bit offset records
     rtz_fused = not (P.level_config(0)["gs"] == 10 and packs[0] in (1, 2))
     waves = tuple(P.level_wavefront(l) for l in range(4))
@@ -636,7 +643,7 @@ def b200_arm(args, rank, world, local_rank):
             mixed["rhs_uniform"] = mixed_vs_fp64(P, uniform_rhs(nrow, f"cuda:{dev}"), lib_stream, args.mixed_tol)
         # the floor of the time ratio: the two forms' algorithmic bytes per
         # iteration (both bandwidth-bound at about the same efficiency)
-        packs = tuple(P.level_pack_width(l) for l in range(4))
+        packs = tuple(column_form(P, l) for l in range(4))
         b64 = metrics.iteration_bytes(n, n, n, vb=8, pack=packs, rtz_fused=rtz_fused, wave=waves)
         b32 = metrics.iteration_bytes(n, n, n, vb=4, pack=packs)
         mixed["byte_floor_ratio"] = round(b32 / b64, 4)
@@ -668,15 +675,14 @@ def b200_arm(args, rank, world, local_rank):
     if rank == 0:
         peak, peak_kind = measured_peak_hbm()
         gs_cfg = tuning[0]["gs"]
-        pack0 = P.level_pack_width(0)
-        gs_pack = pack0 if gs_cfg == 10 else 0
+        pack0 = column_form(P, 0)
+        gs_pack = pack0 if gs_cfg in (10, 11) else 0
         mv_pack = pack0 if tuning[0]["spmv"] == 7 else 0
-        gs_packed = gs_pack > 0
         gs_bytes = metrics.gs_phase_bytes(gs_rows, nrow, pack=gs_pack)
         achieved = gs_bytes / (gs_ms * 1e-3) / 1e9 if gs_ms > 0 else None
         kernel = (f"k_gs_bulk<double,double,false> (level 0, configuration {gs_cfg}"
-                  f"{', packed columns, ' + COLUMN_FORMS[gs_pack] if gs_pack else ''})" if gs_cfg == 10 else
-                  f"k_gs_phase<double,double,false> (level 0, configuration {gs_cfg})")
+                  f"{', ' + COLUMN_FORMS[gs_pack] if gs_pack else ''})" if gs_cfg == 10 else
+                  f"{'k_gs_geo' if gs_cfg == 11 else 'k_gs_phase'}<double,double,false> (level 0, configuration {gs_cfg})")
         tr = committed_traffic()
         traffic = None
         if (tr and tr.get("n") == n and tr.get("config") == gs_cfg and int(tr.get("pack", 0)) == gs_pack
@@ -736,7 +742,7 @@ def b200_arm(args, rank, world, local_rank):
                 "restrict_l0": round(rs_ms / (args.iters * args.steps), 3),
                 "gs_sweeps_l0": round(ws_ms / (args.iters * args.steps), 3) if wave_line else 0.0,
                 "iteration": round(ms / (args.iters * args.steps), 3)},
-            "gpu_launches": gpu_launches_per_set(args.iters, rtz_pass=gs_packed and gs_pack != 3,
+            "gpu_launches": gpu_launches_per_set(args.iters, rtz_pass=gs_pack in (1, 2),
                                                  wave=waves) * args.steps,
             "clocks": clk,
         }
