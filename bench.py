@@ -720,7 +720,7 @@ def b200_arm(args, rank, world, local_rank):
                                    "default path (e2e runs it)"},
             "iteration": {"bytes": bytes_iter, "gbs": round(hbm_gbs, 1), "frac": round(hbm_gbs / peak, 4),
                           "model": "metrics.iteration_bytes: every kernel of a CG iteration streaming its data "
-                                   "once, each level's column index as stored",
+                                   "once, each level's column index as read",
                           "column_form": list(packs),
                           "compulsory_4byte_index_bytes": metrics.compulsory_bytes(n, n, n)},
             "packed_index_bytes": [P.level_packed(l) for l in range(4)],
