@@ -115,9 +115,14 @@ int tune_lanes(hpcg_b200_problem* P, MultiState* m) {
   const char* force = std::getenv("HPCG_B200_MULTI_LANES");
   const char* force_bulk = std::getenv("HPCG_B200_MULTI_BULK");
   const bool have_maps = bulk_maps(P->lev[0]) != nullptr;
+  // form 3: grid columns on every level; above the coarsest the injected rows are
+  // the all-even points and, in the stored order, one run (a run alone may be
+  // another colour's, whose columns k_restrict_m_geo's block does not give)
   bool geo = have_maps;
-  for (int l = 0; l < P->nlev; ++l)
-    geo = geo && P->lev[l].geo_cols && bulk_maps(P->lev[l]) && (l + 1 == P->nlev || P->lev[l].tf_run >= 0);
+  for (int l = 0; l < P->nlev; ++l) {
+    const Level& L = P->lev[l];
+    geo = geo && L.geo_cols && bulk_maps(L) && (l + 1 == P->nlev || (L.geo_f2c && L.tf_run >= 0));
+  }
   if ((force && *force) || (force_bulk && *force_bulk)) {
     const int f = force && *force ? std::atoi(force) : 1;
     m->lanes = f >= 4 && K >= 8 ? 4 : f >= 2 && K >= 4 ? 2 : 1;
