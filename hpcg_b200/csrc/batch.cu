@@ -1318,7 +1318,7 @@ int build_form1(hpcg_b200_batch* B) {
       B->tail_smem = std::max(B->tail_smem, smem);
     }
   }
-  HB_TRY(tail_attributes((const void*)k_b_tail, B->tail_smem));
+  HB_TRY(tail_attributes((const void*)k_b_tail));
   HB_TRY(alloc_copy(B, (void**)&B->geo_items, W.items.data(), sizeof(BGeo) * W.items.size()));
   HB_TRY(alloc_copy(B, (void**)&B->geo_tiles, W.tiles.data(), sizeof(BGeoTile) * W.tiles.size()));
   HB_TRY(alloc_copy(B, (void**)&B->prolong_items, W.res.data(), sizeof(BRes) * W.res.size()));

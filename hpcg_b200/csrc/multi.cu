@@ -292,7 +292,7 @@ int tail_m(hpcg_b200_problem* P, MultiState* m, int l, const double* r, double* 
   static std::atomic<uint64_t> done{0};
   const uint64_t bit = 1ull << c->device;
   if (!(done.load(std::memory_order_acquire) & bit)) {
-    HB_TRY(tail_attributes((const void*)k, 200 * 1024));
+    HB_TRY(tail_attributes((const void*)k));
     done.fetch_or(bit, std::memory_order_release);
   }
   cudaLaunchConfig_t cfg;

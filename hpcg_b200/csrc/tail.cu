@@ -144,7 +144,7 @@ bool launch(hpcg_b200_problem* p, int l, int nlev, const T* rhs, T* x, bool step
   static std::atomic<uint64_t> attr_set{0};
   const uint64_t bit = 1ull << c->device;
   if (!(attr_set.load(std::memory_order_acquire) & bit)) {
-    if (tail_attributes((const void*)k, kMaxSmem) != HPCG_B200_OK) return false;
+    if (tail_attributes((const void*)k) != HPCG_B200_OK) return false;
     attr_set.fetch_or(bit, std::memory_order_release);
   }
   cudaLaunchConfig_t cfg;
@@ -212,8 +212,8 @@ int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<double>* D, size_t
 int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<float>* D, size_t* smem) {
   return describe(p, l, nlev, D, smem);
 }
-int tail_attributes(const void* kernel, size_t smem) {
-  HB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+int tail_attributes(const void* kernel) {
+  HB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
   HB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return HPCG_B200_OK;
 }
