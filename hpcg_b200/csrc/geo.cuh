@@ -39,7 +39,8 @@ struct GeoPhase {
   int hx, hy, hz;   // half-sides
   int ex, ey;       // what the half-sides of the other x / y parity have more
   FastDiv dx, dy;   // by hx, hy
-  int shared;       // whether 32 bytes of a vector may hold rows of two colours
+  int shared;       // whether 32 bytes of a vector may hold rows of two colours, or rows
+                    // and the zero sink behind the last one (which border rows of every colour read)
   uint32_t low[3], high[3];  // slots that leave the grid at the first / last xx, yy, zz
 };
 
@@ -84,7 +85,7 @@ inline GeoPhase geo_phase(const ColourGrid& g, int s) {
   }
   p.start = g.start[s];
   p.shared = 0;
-  for (int u = 0; u < kColours; ++u) p.shared |= g.start[u] % 8 != 0;
+  for (int u = 0; u <= kColours; ++u) p.shared |= g.start[u] % 8 != 0;  // (start[kColours]: the sink)
   p.hx = h[0];
   p.hy = h[1];
   p.hz = h[2];
