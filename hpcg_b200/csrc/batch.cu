@@ -133,10 +133,12 @@ using BatchShape = GsShape<float, kPackGeo>;
 constexpr int kGeoCache = 24;
 
 // A full-slot phase: the single-problem FP32 phase's pipeline and shape. Items
-// item0 .. item0 + nitems - 1.
+// item0 .. item0 + nitems - 1. fence: whether 32 bytes of a vector of one of them
+// may hold rows of two colours (griddep_wait): sides are multiples of 16, so that is
+// so on level 3, where they are multiples of 2.
 __global__ void __launch_bounds__(BatchShape::threads, 1)
     k_b_gs_geo(const BGeo* __restrict__ items, int item0, int nitems, const BGeoTile* __restrict__ tiles, int ntiles,
-               const BScal* __restrict__ sc, unsigned* fault) {
+               const BScal* __restrict__ sc, unsigned* fault, int fence) {
   __shared__ BGeo cache[kGeoCache];
   const int words = min(nitems, kGeoCache) * (int)(sizeof(BGeo) / sizeof(int));
   for (int i = threadIdx.x; i < words; i += blockDim.x)
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(BatchShape::threads, 1)
         else
           work(items[item0 + at]);
       },
-      fault, false);  // (sides are multiples of 16: colours start on whole sectors)
+      fault, fence != 0);
 }
 
 // A first-sweep phase (k_gs_first_geo's arithmetic), 256 rows a tile.
@@ -812,6 +814,7 @@ struct GeoStep {
   int ntiles;
   int item_off;  // kFull: first item, items
   int nitems;
+  int shared;    // kFull: whether an item's colours may meet in 32 bytes (GeoPhase::shared)
 };
 
 }  // namespace
@@ -972,11 +975,11 @@ void build_geo(hpcg_b200_batch* B, int l, GeoLists& W) {
   if (in.empty() || l >= kMaxLevels) {  // the others' levels are done above: now the small ones of all
     bool any = false;
     for (int p = 0; p < m; ++p) any = any || B->tail_at[p] < B->probs[p]->nlev;
-    if (any) B->geo_steps.push_back(GeoStep{GeoStep::kTail, 0, 0, 0, 0, 0});
+    if (any) B->geo_steps.push_back(GeoStep{GeoStep::kTail, 0, 0, 0, 0, 0, 0});
     return;
   }
   auto step = [&](GeoStep::Kind kind, int s, int rows) {
-    GeoStep st{kind, s, (int)W.tiles.size(), 0, (int)W.items.size(), (int)in.size()};
+    GeoStep st{kind, s, (int)W.tiles.size(), 0, (int)W.items.size(), (int)in.size(), 0};
     for (int p : in) {
       const Level& L = B->probs[p]->lev[l];
       const int item = (int)W.items.size();
@@ -991,6 +994,7 @@ void build_geo(hpcg_b200_batch* B, int l, GeoLists& W) {
       it.sink = sink_of(L);
       it.prob = p;
       it.geo = L.geo_cols->block[s];
+      st.shared |= it.geo.shared;
       W.items.push_back(it);
       // whole-block tiles for the copies, from the first row for the others
       const int first = kind == GeoStep::kFull ? it.r0 / rows * rows : it.r0;
@@ -1009,7 +1013,7 @@ void build_geo(hpcg_b200_batch* B, int l, GeoLists& W) {
   if (l + 1 < kMaxLevels) {
     step(GeoStep::kRestrict, kColours - 1, kTile);
     build_geo(B, l + 1, W);
-    GeoStep st{GeoStep::kProlong, 0, (int)W.rtiles.size(), 0, 0, 0};
+    GeoStep st{GeoStep::kProlong, 0, (int)W.rtiles.size(), 0, 0, 0, 0};
     for (int p : in) {
       const Level& L = B->probs[p]->lev[l];
       const Level& C = B->probs[p]->lev[l + 1];
@@ -1080,7 +1084,7 @@ int launch_geo_step(hpcg_b200_batch* B, const GeoStep& st) {
       attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attr[0].val.programmaticStreamSerializationAllowed = 1;
       HB_CK(cudaLaunchKernelEx(&cfg, k_b_gs_geo, (const BGeo*)B->geo_items, st.item_off, st.nitems, tiles, st.ntiles,
-                               (const BScal*)B->sc, c->fault));
+                               (const BScal*)B->sc, c->fault, st.shared));
       return HPCG_B200_OK;
     }
     case GeoStep::kFirst:
