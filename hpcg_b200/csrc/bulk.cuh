@@ -329,6 +329,12 @@ __device__ __forceinline__ uint64_t evict_first_policy() {
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
+// Before a block's first use of a tensor map that lies in global memory (not in the
+// kernel's parameters): the map is read through a proxy of its own, which may still
+// hold what an earlier map at the same address said.
+__device__ __forceinline__ void tensormap_acquire(const CUtensorMap* m) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(m) : "memory");
+}
 // Programmatic dependent launch: a kernel launched with programmatic stream
 // serialization may start while the kernel before it on the stream finishes;
 // griddep_wait() returns once that kernel has completed and its writes are in the
@@ -557,6 +563,7 @@ __device__ __forceinline__ void bulk_tiles_driven(int ntiles, Src src, Skip skip
       for (int s = 0; s < S; ++s) last[s] = -1;
       int i = 0, ends = 0;
       bool ok = true;
+      const CUtensorMap* seen = nullptr;  // the map last acquired (a list goes matrix by matrix)
       for (int tile = blockIdx.x; ok && ends < G; tile += gridDim.x) {
         const bool end = tile >= ntiles;
         if (!end && skip(tile)) continue;
@@ -582,10 +589,12 @@ __device__ __forceinline__ void bulk_tiles_driven(int ntiles, Src src, Skip skip
           first[s] = ts.q0;
           mbar_expect_tx(&full[s], Shape::value_bytes);
           T* sv = reinterpret_cast<T*>(smem + s * SB);
-          if constexpr (bulk_whole_tile<T>())
+          if constexpr (bulk_whole_tile<T>()) {
             bulk_g2s(sv, ts.vals, Shape::value_bytes, &full[s], policy);
-          else
+          } else {
+            if (ts.map != seen) tensormap_acquire(seen = ts.map);
             tma_load_2d(sv, ts.map, (int)(unsigned)ts.q0, 0, &full[s], policy);
+          }
 #pragma unroll
           for (int u = 0; u < S; ++u)
             if (u == s) last[u] = use;

@@ -31,3 +31,22 @@ def test_batches_side_by_side(binding, later, first):
     finally:
         for B in live:
             B.free()
+
+
+def test_batches_one_after_another(binding, monkeypatch):
+    """Batches whose matrices (and their tensor maps) take the memory that a freed
+    batch of other grids gave back: the register kernels' bits, which use no maps."""
+    lists = [[(64, 32, 48), (32, 32, 32)], [(32, 48, 64), (48, 16, 32)], [(16, 16, 16)], [(64, 32, 48), (32, 32, 32)]]
+    got = {}
+    for bulk in ("0", "1"):
+        monkeypatch.setenv("HPCG_B200_BATCH_BULK", bulk)
+        got[bulk] = []
+        for dims in lists:
+            B = binding.Batch(dims)
+            try:
+                got[bulk].append(solve(B))
+            finally:
+                B.free()
+    for a, b in zip(got["0"], got["1"]):
+        for x, y in zip(a, b):
+            assert np.array_equal(x, y)
