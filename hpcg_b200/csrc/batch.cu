@@ -1075,16 +1075,12 @@ int launch_geo_step(hpcg_b200_batch* B, const GeoStep& st) {
     case GeoStep::kFull: {
       static std::atomic<uint64_t> attr_set{0};  // devices on which the shared-memory size is enabled
       bulk_attr(k_b_gs_geo, BatchShape::smem, c->device, &attr_set);
-      cfg.gridDim = dim3(std::max(1, std::min(st.ntiles, c->sms)));
-      cfg.blockDim = dim3(BatchShape::threads);
-      cfg.dynamicSmemBytes = BatchShape::smem;
       // early launch: the producer reads values and, for the tiles to skip, the
       // convergence flags, which are written before a plainly launched kernel
       // (a first-sweep phase, a prolongation) of every V-cycle
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      HB_CK(cudaLaunchKernelEx(&cfg, k_b_gs_geo, (const BGeo*)B->geo_items, st.item_off, st.nitems, tiles, st.ntiles,
-                               (const BScal*)B->sc, c->fault, st.shared));
+      HB_CK(launch_early(c->stream, k_b_gs_geo, std::max(1, std::min(st.ntiles, c->sms)), BatchShape::threads,
+                         BatchShape::smem, B->geo_items, st.item_off, st.nitems, tiles, st.ntiles, B->sc, c->fault,
+                         st.shared));
       return HPCG_B200_OK;
     }
     case GeoStep::kFirst:

@@ -252,20 +252,10 @@ int launch_phase_m_geo(Context* c, const Level& L, const double* rhs, double* x,
   auto k = k_gs_phase_m_geo<K>;
   static std::atomic<uint64_t> done{0};
   bulk_attr(k, Sh::smem, c->device, &done);
-  cudaLaunchConfig_t cfg;
-  std::memset(&cfg, 0, sizeof(cfg));
   const int64_t tiles = ((int64_t)r1 - (r0 & ~(kBulkRows - 1)) + kBulkRows - 1) / kBulkRows;
-  cfg.gridDim = dim3((unsigned)std::min<int64_t>(tiles, 2 * c->sms));
-  cfg.blockDim = dim3(Sh::threads);
-  cfg.dynamicSmemBytes = Sh::smem;
-  cfg.stream = c->stream;
-  cudaLaunchAttribute attr[1];  // the producer reads the matrix only (see k_gs_bulk)
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  HB_CK(cudaLaunchKernelEx(&cfg, k, (const double*)L.val, L.pitch, rhs, x, r0, r1, c->fault, bulk_maps(L)->val,
-                           sink_of(L), geo));
+  // early: the producer reads the matrix only (see k_gs_bulk)
+  HB_CK(launch_early(c->stream, k, (int)std::min<int64_t>(tiles, 2 * c->sms), Sh::threads, Sh::smem, L.val, L.pitch,
+                     rhs, x, r0, r1, c->fault, bulk_maps(L)->val, sink_of(L), geo));
   return HPCG_B200_OK;
 }
 
