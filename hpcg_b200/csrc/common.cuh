@@ -251,6 +251,7 @@ struct Level {
   // the level's colour blocks as the kernels that take the columns from the grid
   // read them (geo.cuh; host memory), nullptr where they read stored columns
   GeoGrid* geo_cols = nullptr;
+  bool mv_rule = false;  // the SpMV's configuration is the rule's, named or timed by nobody
   double* valt = nullptr;  // FP64 values in the layout tail.cuh reads (small levels only, built on first use)
 };
 

@@ -915,9 +915,10 @@ void rule_config32(Level& L) {
     L.gs_first32_at[s] = large && s == kColours - 1 ? kBulkCfg : L.gs_first32;
 }
 
-int autotune(hpcg_b200_problem* P) {
+// small: also decide which small levels run in one launch (not for an SpMV alone).
+int autotune(hpcg_b200_problem* P, bool small = true) {
   Context* c = P->ctx;
-  tail_first(P, false);  // may allocate: before any capture
+  if (small) tail_first(P, false);  // may allocate: before any capture
   const char* force = std::getenv("HPCG_B200_CONFIG");
   for (int l = 0; l < P->nlev; ++l) {
     Level& L = P->lev[l];
@@ -950,7 +951,10 @@ int autotune(hpcg_b200_problem* P) {
         HB_TRY(ensure_wavefront(L));
         L.wf = L.wf_tpu > 0 ? 1 : 0;
       }
-      if (wave_force() >= 0) continue;
+      if (wave_force() >= 0) {
+        L.mv_rule = !(fo && *fo);
+        continue;
+      }
     }
     double* xs = l == 0 ? P->Ap : L.x;
     double* rs = l == 0 ? P->zprev : L.r;
@@ -1769,7 +1773,8 @@ int device_view(Context* c, const double* v, int n, int slot, const double** out
 // place (k_spmv_nat) instead of permuting them around the bulk-copy SpMV: 96^3 47
 // against 57 us, 128^3 89 against 104, 192^3 312 against 323. Beyond, x no longer
 // stays in the L2 from one colour block to the next, which the slab order of the
-// bulk-copy SpMV provides for.
+// bulk-copy SpMV provides for. Where the environment names the level's configurations
+// or asks for timed ones, the call runs what it named (Level::mv_rule).
 constexpr int kNatSpmv = 1 << 23;
 
 // whether two runs of n doubles share memory
@@ -1814,8 +1819,9 @@ int hpcg_b200_spmv(hpcg_b200_problem* p, const double* x, double* y) {
   Setter dev(p->device);
   const Level& L = p->lev[0];
   Context* c = p->ctx;
+  HB_TRY(autotune(p, false));
   bool xdev = false, ydev = false;
-  if (L.geo_cols && L.n <= kNatSpmv) {
+  if (L.geo_cols && L.mv_rule && L.n <= kNatSpmv) {
     HB_TRY(locate_ptr(x, p->device, &xdev, "input vector"));
     HB_TRY(locate_ptr(y, p->device, &ydev, "output vector"));
     if (xdev && ydev && !overlap(x, y, L.n)) {
@@ -1829,7 +1835,6 @@ int hpcg_b200_spmv(hpcg_b200_problem* p, const double* x, double* y) {
     }
   }
   HB_TRY(load_vector(p, 0, x, p->p));
-  HB_TRY(autotune(p));
   spmv_dispatch<double, false>(c, L, L.val, p->p, p->Ap, nullptr);
   HB_CK(cudaGetLastError());
   return store_vector(p, 0, p->Ap, y);
