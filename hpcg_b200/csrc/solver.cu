@@ -1777,10 +1777,10 @@ int device_view(Context* c, const double* v, int n, int slot, const double** out
 // or asks for timed ones, the call runs what it named (Level::mv_rule).
 constexpr int kNatSpmv = 1 << 23;
 
-// whether two runs of n doubles share memory
-bool overlap(const double* a, const double* b, int64_t n) {
-  const uintptr_t u = (uintptr_t)a, v = (uintptr_t)b, bytes = sizeof(double) * (uintptr_t)n;
-  return u < v + bytes && v < u + bytes;
+// whether runs of na doubles at a and nb at b share memory
+bool overlap(const double* a, int64_t na, const double* b, int64_t nb) {
+  const uintptr_t u = (uintptr_t)a, v = (uintptr_t)b;
+  return u < v + sizeof(double) * (uintptr_t)nb && v < u + sizeof(double) * (uintptr_t)na;
 }
 
 // The result of lone reduction `call` once the GPU has stored it: the host looks
@@ -1824,7 +1824,7 @@ int hpcg_b200_spmv(hpcg_b200_problem* p, const double* x, double* y) {
   if (L.geo_cols && L.mv_rule && L.n <= kNatSpmv) {
     HB_TRY(locate_ptr(x, p->device, &xdev, "input vector"));
     HB_TRY(locate_ptr(y, p->device, &ydev, "output vector"));
-    if (xdev && ydev && !overlap(x, y, L.n)) {
+    if (xdev && ydev && !overlap(x, L.n, y, L.n)) {
       FastDiv dx, dy;
       dx.init((unsigned)L.g.nx);
       dy.init((unsigned)L.g.ny);
@@ -1920,13 +1920,18 @@ int hpcg_b200_adjoint(hpcg_b200_problem* p, const double* x, const double* g, in
   HB_TRY(run_cg(p, max_iter, tolerance, true, niters, &nr, &nr0, nullptr));
   HB_TRY(store_vector(p, 0, p->x, grad_b));  // dL/db = lambda
   // on grid columns the gradients are formed from the natural-order vectors:
-  // lambda as just stored, x as given, or their device copies
-  bool xdev = false, bdev = false;
+  // lambda as just stored, x as given, or their device copies; from the problem's
+  // own colour-order vectors where the gradients go over one of those
+  bool xdev = false, bdev = false, dev_out = false;
   HB_TRY(locate_ptr(x, p->device, &xdev, "x"));
   HB_TRY(locate_ptr(grad_b, p->device, &bdev, "grad_b"));
+  HB_TRY(locate_ptr(grad_values27, p->device, &dev_out, "grad_values27"));
   const double* xn = x;
   const double* ln = bdev ? grad_b : c->stage[1];
-  if (!L.geo_cols) {
+  const int64_t entries = (int64_t)kSlots * L.n;
+  const bool natural = L.geo_cols && !(dev_out && ((xdev && overlap(grad_values27, entries, x, L.n)) ||
+                                                   (bdev && overlap(grad_values27, entries, grad_b, L.n))));
+  if (!natural) {
     HB_TRY(load_vector(p, 0, x, p->Ap));  // the forward solution, colour order
   } else if (!xdev) {
     if (bdev) HB_TRY(ensure_stage(c, L.n));  // (else stage[1] holds lambda and they are large enough)
@@ -1934,11 +1939,9 @@ int hpcg_b200_adjoint(hpcg_b200_problem* p, const double* x, const double* g, in
     xn = c->stage[0];
   }
   double* out = grad_values27;
-  bool dev_out = false;
-  HB_TRY(locate_ptr(grad_values27, p->device, &dev_out, "grad_values27"));
-  const size_t bytes = sizeof(double) * kSlots * (size_t)L.n;
+  const size_t bytes = sizeof(double) * (size_t)entries;
   if (!dev_out) HB_CK(cudaMalloc(&out, bytes));
-  if (L.geo_cols) {
+  if (natural) {
     FastDiv dx, dy;
     dx.init((unsigned)L.g.nx);
     dy.init((unsigned)L.g.ny);
