@@ -1081,6 +1081,9 @@ int mg32_level(hpcg_b200_problem* p, int l, const float* r, float* x);
 // Runs `direct` (launches on c's stream, the same ones every time) as one graph
 // launch once it has been captured into ex; inside a capture, with graphs off
 // or refused, in the natural-order mode and under the launch profiler directly.
+// The capture is on a stream of its own, through a copy of the context that only
+// this problem sees: the context's stream is every problem's on the GPU, and a call
+// of another thread would be recorded into the graph, or end the capture by waiting.
 template <typename F>
 int run_captured(hpcg_b200_problem* p, cudaGraphExec_t& ex, F&& direct) {
   Context* c = p->ctx;
@@ -1090,12 +1093,26 @@ int run_captured(hpcg_b200_problem* p, cudaGraphExec_t& ex, F&& direct) {
       p->symgs_mode != HPCG_B200_SYMGS_COLOUR)
     return direct();
   if (!ex) {
-    HB_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    const int st = direct();
+    Context rec;
+    rec.device = c->device;
+    rec.sms = c->sms;
+    rec.partials = c->partials;
+    rec.scal = c->scal;
+    rec.scal_host = c->scal_host;
+    rec.fault = c->fault;
+    HB_CK(cudaStreamCreateWithFlags(&rec.stream, cudaStreamNonBlocking));
     cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+    int st = HPCG_B200_OK;
+    cudaError_t e = cudaStreamBeginCapture(rec.stream, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      p->ctx = &rec;
+      st = direct();
+      p->ctx = c;
+      e = cudaStreamEndCapture(rec.stream, &g);
+    }
     if (st == HPCG_B200_OK && e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
     if (g) cudaGraphDestroy(g);
+    cudaStreamDestroy(rec.stream);
     if (st != HPCG_B200_OK || e != cudaSuccess) {  // refused: stream launches from now on
       cudaGetLastError();
       ex = nullptr;
