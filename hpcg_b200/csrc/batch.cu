@@ -1300,25 +1300,27 @@ int build_form1(hpcg_b200_batch* B) {
   int cut = 0;
   for (hpcg_b200_problem* p : B->probs)
     cut = std::max(cut, tail_first_within(p, true, kBatchTailRows, B->m > 8 ? 110 * 1024 : 200 * 1024));
+  std::vector<TailDesc<float>> descs(B->m);
+  for (;; ++cut) {
+    B->tail_cluster = 1;
+    B->tail_smem = 0;
+    bool any = false;
+    for (int p = 0; p < B->m; ++p) {
+      hpcg_b200_problem* P = B->probs[p];
+      std::memset(&descs[p], 0, sizeof(descs[p]));
+      if (cut >= P->nlev) continue;
+      any = true;
+      size_t smem = 0;
+      B->tail_cluster = std::max(B->tail_cluster, tail_desc(P, cut, P->nlev - cut, &descs[p], &smem));
+      B->tail_smem = std::max(B->tail_smem, smem);
+    }
+    if (!any || tail_fits((const void*)k_b_tail, B->tail_cluster, B->tail_smem)) break;
+  }
   B->tail_at.assign(B->m, cut);
   GeoLists W;
   build_geo(B, 0, W);
-  std::vector<TailDesc<float>> descs(B->m);
   std::vector<GeoGrid> grids;
-  B->tail_cluster = 1;
-  B->tail_smem = 0;
-  for (int p = 0; p < B->m; ++p) {
-    hpcg_b200_problem* P = B->probs[p];
-    grids.push_back(*P->lev[0].geo_cols);
-    std::memset(&descs[p], 0, sizeof(descs[p]));
-    const int l = B->tail_at[p];
-    if (l < P->nlev) {
-      size_t smem = 0;
-      B->tail_cluster = std::max(B->tail_cluster, tail_desc(P, l, P->nlev - l, &descs[p], &smem));
-      B->tail_smem = std::max(B->tail_smem, smem);
-    }
-  }
-  HB_TRY(tail_attributes((const void*)k_b_tail));
+  for (hpcg_b200_problem* P : B->probs) grids.push_back(*P->lev[0].geo_cols);
   HB_TRY(alloc_copy(B, (void**)&B->geo_items, W.items.data(), sizeof(BGeo) * W.items.size()));
   HB_TRY(alloc_copy(B, (void**)&B->geo_tiles, W.tiles.data(), sizeof(BGeoTile) * W.tiles.size()));
   HB_TRY(alloc_copy(B, (void**)&B->prolong_items, W.res.data(), sizeof(BRes) * W.res.size()));

@@ -18,6 +18,7 @@ struct MultiState {
   int lanes = 1;  // threads per row of the matrix kernels (K/lanes systems each), tuned on creation
   int bulk = 0;   // 0: register-pipelined kernels; 1: bulk-copy full phases and SpMV; 2: first sweep too;
                   // 3: columns from the grid, the small levels in one launch
+  int tail = kMaxLevels;  // form 3: the first of those
   double *b = nullptr, *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *Ap = nullptr;
   double* lr[kMaxLevels] = {nullptr};  // coarse right-hand sides (levels > 0)
   double* lx[kMaxLevels] = {nullptr};  // coarse solutions (levels > 0)
@@ -106,6 +107,19 @@ int time_iteration(hpcg_b200_problem* P, MultiState* m, cudaEvent_t e0, cudaEven
   return HPCG_B200_OK;
 }
 
+// The first level of the one-launch small end in form 3.
+template <int K>
+int tail_first_m(hpcg_b200_problem* P) {
+  int f = tail_first(P, false);
+  for (; f < P->nlev; ++f) {
+    TailDesc<double> D;
+    size_t smem = 0;
+    const int size = tail_desc(P, f, P->nlev - f, &D, &smem);
+    if (tail_fits((const void*)k_tail_m<K>, size, smem)) break;
+  }
+  return f;
+}
+
 // Threads per row and kernel form of the matrix kernels: the fastest V-cycle +
 // SpMV (round-robin repetitions over lanes 1, 2, 4 x register-pipelined, bulk
 // full phases, bulk everywhere), or HPCG_B200_MULTI_LANES / HPCG_B200_MULTI_BULK.
@@ -128,13 +142,13 @@ int tune_lanes(hpcg_b200_problem* P, MultiState* m) {
     m->lanes = f >= 4 && K >= 8 ? 4 : f >= 2 && K >= 4 ? 2 : 1;
     const int b = force_bulk && *force_bulk ? std::atoi(force_bulk) : 0;
     m->bulk = have_maps ? (b < 0 ? 0 : b == 3 && geo ? 3 : b > 2 ? 2 : b) : 0;
-    tail_first(P, false);
+    m->tail = tail_first_m<K>(P);
     return HPCG_B200_OK;
   }
   const char* tune = std::getenv("HPCG_B200_TUNE");
   if (geo && !(tune && *tune && tune[0] != '0')) {
     m->bulk = 3;  // the best form wherever it applies (128^3, eight systems: 42 against 55 ms for 20 iterations)
-    tail_first(P, false);  // may allocate: before any capture
+    m->tail = tail_first_m<K>(P);  // may allocate: before any capture
     return HPCG_B200_OK;
   }
   Context* c = P->ctx;
@@ -279,12 +293,6 @@ int tail_m(hpcg_b200_problem* P, MultiState* m, int l, const double* r, double* 
     D.lev[i].x = m->lx[l + i];
   }
   auto k = k_tail_m<K>;
-  static std::atomic<uint64_t> done{0};
-  const uint64_t bit = 1ull << c->device;
-  if (!(done.load(std::memory_order_acquire) & bit)) {
-    HB_TRY(tail_attributes((const void*)k));
-    done.fetch_or(bit, std::memory_order_release);
-  }
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(size * K);
@@ -420,7 +428,7 @@ template <int K, int LANES, int BULK>
 int mg_m(hpcg_b200_problem* P, MultiState* m, int l, const double* r, double* x) {
   const Level& L = P->lev[l];
   Context* c = P->ctx;
-  if (BULK == 3 && l >= tail_first(P, false)) return tail_m<K>(P, m, l, r, x);
+  if (BULK == 3 && l >= m->tail) return tail_m<K>(P, m, l, r, x);
   HB_TRY((gs_colour_m<K, LANES, BULK>(c, L, r, x, true)));
   if (l + 1 < P->nlev) {
     const Level& C = P->lev[l + 1];
@@ -455,7 +463,7 @@ template <int K, int LANES, int BULK>
 int coarse_m(hpcg_b200_problem* P, MultiState* m) {
   Context* c = P->ctx;
   auto direct = [&]() -> int { return mg_m<K, LANES, BULK>(P, m, 1, m->lr[1], m->lx[1]); };
-  if (BULK == 3 && tail_first(P, false) <= 1) return direct();  // one launch
+  if (BULK == 3 && m->tail <= 1) return direct();  // one launch
   const char* ge = std::getenv("HPCG_B200_GRAPH");
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   HB_CK(cudaStreamIsCapturing(c->stream, &cs));

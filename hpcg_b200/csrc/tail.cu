@@ -135,18 +135,20 @@ int describe(hpcg_b200_problem* p, int l, int nlev, TailDesc<T>* desc, size_t* s
 }
 
 template <typename T>
+bool fits(hpcg_b200_problem* p, int l) {
+  TailDesc<T> D;
+  size_t smem = 0;
+  const int size = describe(p, l, p->nlev - l, &D, &smem);
+  return tail_fits((const void*)k_tail<T>, size, smem);
+}
+
+template <typename T>
 bool launch(hpcg_b200_problem* p, int l, int nlev, const T* rhs, T* x, bool step) {
   Context* c = p->ctx;
   TailDesc<T> D;
   size_t smem = 0;
   const int size = describe(p, l, nlev, &D, &smem);
   auto k = k_tail<T>;
-  static std::atomic<uint64_t> attr_set{0};
-  const uint64_t bit = 1ull << c->device;
-  if (!(attr_set.load(std::memory_order_acquire) & bit)) {
-    if (tail_attributes((const void*)k) != HPCG_B200_OK) return false;
-    attr_set.fetch_or(bit, std::memory_order_release);
-  }
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(size);
@@ -179,7 +181,8 @@ int tail_first(hpcg_b200_problem* p, bool f32) {
   if (first >= 0) return first;
   first = p->nlev;
   if (!wanted()) return first;
-  const int f = first_within(p, f32, max_rows(f32), kMaxSmem);
+  int f = first_within(p, f32, max_rows(f32), kMaxSmem);
+  while (f < p->nlev && !(f32 ? fits<float>(p, f) : fits<double>(p, f))) ++f;
   if (!f32)
     for (int l = f; l < p->nlev; ++l)
       if (!p->lev[l].valt && tail_values(p, l) != HPCG_B200_OK) return first;  // no memory: the phases run
@@ -212,10 +215,28 @@ int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<double>* D, size_t
 int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<float>* D, size_t* smem) {
   return describe(p, l, nlev, D, smem);
 }
-int tail_attributes(const void* kernel) {
-  HB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-  HB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  return HPCG_B200_OK;
+bool tail_fits(const void* kernel, int size, size_t smem) {
+  const char* e = std::getenv("HPCG_B200_TAIL_CLUSTER");
+  if (e && *e && size > std::atoi(e)) return false;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(kTailThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) == cudaSuccess &&
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess)
+    return clusters > 0;
+  cudaGetLastError();
+  return false;
 }
 
 bool tail_step_ok(hpcg_b200_problem* p, int l) {

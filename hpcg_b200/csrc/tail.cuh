@@ -411,12 +411,15 @@ __global__ void __launch_bounds__(kTailThreads, 1)
 
 // Host side (tail.cu). tail_desc: the description of problem p's levels l ..
 // l + nlev - 1, the shared memory of a block; returns the blocks of a cluster (a
-// power of two). tail_attributes: lets a kernel built on tail_run use as much of it
-// as any description asks for: the limit is the kernel's, not a launch's, so one set
-// for one problem's need would refuse a larger problem that is still alive.
+// power of two). tail_fits: whether the GPU can hold one such cluster of a kernel
+// built on tail_run, asked before a launch of it is planned: a refusal would come in
+// the middle of a capture. It lets the kernel use as much shared memory as any
+// description asks for: the limit is the kernel's, not a launch's, so one set for one
+// problem's need would refuse a larger problem that is still alive.
+// HPCG_B200_TAIL_CLUSTER=n: as on a GPU that holds clusters of at most n blocks.
 int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<double>* D, size_t* smem);
 int tail_desc(hpcg_b200_problem* p, int l, int nlev, TailDesc<float>* D, size_t* smem);
-int tail_attributes(const void* kernel);
+bool tail_fits(const void* kernel, int size, size_t smem);
 // tail_first for other bounds than the single problem's: rows of a block in one
 // phase, bytes of its shared memory
 int tail_first_within(const hpcg_b200_problem* p, bool f32, int64_t rows, int64_t bytes);
