@@ -455,7 +455,7 @@ def mixed_vs_fp64(P, b, lib_stream, tol, max_iter=2000, profile_iters=20):
     peak, _ = measured_peak_hbm()
     pack = column_form(P, 0) if P.level_config(0)["gs32"] in (10, 11) else 0
     full_gbs = metrics.gs_phase_bytes(fu_rows, n, vb=4, pack=pack) / (fu_ms * 1e-3) / 1e9 if fu_ms else None
-    first_gbs = metrics.first_sweep_bytes(fi_rows, vb=4) / (fi_ms * 1e-3) / 1e9 if fi_ms else None
+    first_gbs = metrics.first_sweep_bytes(fi_rows, vb=4, pack=column_form(P, 0)) / (fi_ms * 1e-3) / 1e9 if fi_ms else None
     return {"fp64": {"iters": it64, "seconds": round(t64, 3), "scaled_residual": nr64 / nr064},
             "fp32_vcycle": {"iters": it32, "seconds": round(t32, 3), "scaled_residual": nr32 / nr032,
                             "true_residual": res},
@@ -468,7 +468,7 @@ def mixed_vs_fp64(P, b, lib_stream, tol, max_iter=2000, profile_iters=20):
                 "first_ms_per_iter": round(fi_ms / profile_iters, 3),
                 "first_gbs": round(first_gbs, 1) if first_gbs else None,
                 "bytes_per_row": {"full": round(metrics.gs_phase_bytes(1, 8, vb=4, pack=pack), 3),
-                                  "first_sweep": 130},
+                                  "first_sweep": metrics.first_sweep_bytes(1, 4, column_form(P, 0))},
                 "column_form": pack}}
 
 
@@ -734,7 +734,7 @@ def b200_arm(args, rank, world, local_rank):
             "spmv": {"launches": sp_launch, "avg_ms": round(sp_ms / max(sp_launch, 1), 4),
                      "gbs": round(metrics.spmv_bytes(sp_rows, pack=mv_pack) / (sp_ms * 1e-3) / 1e9, 1)
                      if sp_ms else None, "column_form": mv_pack},
-            "first_sweep_gbs": round(metrics.first_sweep_bytes(gf_rows) / (gf_ms * 1e-3) / 1e9, 1) if gf_ms else None,
+            "first_sweep_gbs": round(metrics.first_sweep_bytes(gf_rows, pack=packs[0]) / (gf_ms * 1e-3) / 1e9, 1) if gf_ms else None,
             "kernel_ms_per_iter": {
                 "gs_full_l0": round(phase_ms / (args.iters * args.steps), 3),
                 "gs_first_l0": round(gf_ms / (args.iters * args.steps), 3),

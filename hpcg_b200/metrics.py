@@ -133,14 +133,15 @@ def spmv_bytes(rows, vb=8, pack=0):
     return rows * (SLOTS * vb + index_bytes_per_row(pack) + 2 * vb)
 
 
-def first_sweep_bytes(rows, vb=8):
+def first_sweep_bytes(rows, vb=8, pack=0):
     """Algorithmic bytes of the first forward sweeps (x = 0) that together
     updated `rows` rows, summed over whole sweeps (all eight colours): a phase
     reads only the slots of colours swept before it, 13 of the 27 per row on
     average (each neighbouring pair of colours once: 8 colours x 26 neighbours
-    / 2 / 8), plus the diagonal value, the right-hand side, the x write and the
+    / 2 / 8), each with its int32 column unless the level's columns come from the
+    grid (pack 4), plus the diagonal value, the right-hand side, the x write and the
     swept colours' x (28 colour-eighths over 8 phases = 3.5 entries per row)."""
-    return rows * (13 * (vb + 4) + vb + 2 * vb + 3.5 * vb)
+    return rows * (13 * (vb + (0 if pack == 4 else 4)) + vb + 2 * vb + 3.5 * vb)
 
 
 
@@ -155,7 +156,7 @@ def iteration_bytes(nx, ny, nz, vb=8, pack=(1, 1, 1, 1), nlevels=4, parts=False,
     (8 in the FP64 form, 4 in the FP32 V-cycle):
 
     * pre-smoother: the first forward sweep from x = 0 (first_sweep_bytes,
-      13 slots with int32 columns on average) and the backward sweep's 7
+      13 slots on average, with int32 columns unless pack[l] is 4) and the backward sweep's 7
       phases, 7/8 N_l F_l (the colour at the turn is not recomputed);
     * residual + restriction (levels above the coarsest): N_l/8 coarse rows of
       27 vb + I_l + 2 vb + 4 (rf read, rc written, the coarse row's index) and
@@ -186,7 +187,7 @@ def iteration_bytes(nx, ny, nz, vb=8, pack=(1, 1, 1, 1), nlevels=4, parts=False,
         wl = l < len(wave) and wave[l]
         # a sweep that starts from nonzero x and updates the fraction f of the rows
         sweep = (lambda f: f * n_l * (29.0 * vb + ib) + n_l * vb) if wl else (lambda f: f * n_l * full)
-        b = first_sweep_bytes(n_l, vb) + sweep(7.0 / 8.0)
+        b = first_sweep_bytes(n_l, vb, pack[l]) + sweep(7.0 / 8.0)
         if l < nlevels - 1:
             b += n_l / 8.0 * (27.0 * vb + ib + 2.0 * vb + 4.0) + n_l * vb
             b += n_l / 8.0 * (8.0 + 3.0 * vb)
