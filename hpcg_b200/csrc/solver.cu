@@ -891,25 +891,26 @@ void pick_first(const float (&t)[kColours][kGsConfigs], int (&at)[kColours], int
 //    stream (384^3: 1.04 ms; 128^3: 43 us, in storage order 41).
 constexpr int kBeyondL2 = 4 << 20;  // rows: 32 MB a vector, 900 MB of values
 
-constexpr int kGeoRows = 2 * 2 * 148 * kThreads;  // rows of a phase: two rounds of two blocks of k_gs_geo on an SM
+// rows of a phase: two rounds of two blocks of k_gs_geo on each SM (148: 151552)
+int geo_rows(const Context* c) { return 2 * 2 * c->sms * kThreads; }
 
 bool by_rule(const Level& L) {
   const char* e = std::getenv("HPCG_B200_TUNE");
   return L.geo_cols && !(e && *e && e[0] != '0');
 }
 
-void rule_config(Level& L) {
+void rule_config(const Context* c, Level& L) {
   const bool large = L.n >= kBeyondL2;
-  L.gs_sched = L.n / kColours <= kGeoRows ? kGeoCfg : kBulkCfg;
+  L.gs_sched = L.n / kColours <= geo_rows(c) ? kGeoCfg : kBulkCfg;
   L.gs_first = kGeoCfg;
   for (int s = 0; s < kColours; ++s) L.gs_first_at[s] = large && s == kColours - 1 ? kBulkCfg : kGeoCfg;
   L.mv_sched = kBulkMvCfg;
   L.mv_order = large ? 2 : 0;
 }
 
-void rule_config32(Level& L) {
+void rule_config32(const Context* c, Level& L) {
   const bool large = L.n >= kBeyondL2;
-  L.gs_sched32 = L.n / kColours <= kGeoRows ? kGeoCfg : kBulkCfg;
+  L.gs_sched32 = L.n / kColours <= geo_rows(c) ? kGeoCfg : kBulkCfg;
   L.gs_first32 = large ? kGeoCfg + 1 : kGeoCfg;
   for (int s = 0; s < kColours; ++s)
     L.gs_first32_at[s] = large && s == kColours - 1 ? kBulkCfg : L.gs_first32;
@@ -944,7 +945,7 @@ int autotune(hpcg_b200_problem* P, bool small = true) {
       continue;
     }
     if (by_rule(L)) {
-      rule_config(L);
+      rule_config(c, L);
       const char* fo = std::getenv("HPCG_B200_SPMV_ORDER");
       if (fo && *fo) L.mv_order = std::atoi(fo);
       if (wave_force() > 0) {
@@ -1440,7 +1441,7 @@ int ensure_f32(hpcg_b200_problem* P) {
         continue;
       }
       if (by_rule(L)) {
-        rule_config32(L);
+        rule_config32(c, L);
         continue;
       }
       const int r0 = L.g.start[1], r1 = L.g.start[2];
