@@ -22,6 +22,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -379,10 +380,18 @@ struct Context {
   unsigned* lone_count = nullptr;
   void* lone = nullptr;
   std::atomic<unsigned long long> lone_call{0};
+  // streams that captures record on, between two uses (take_recorder)
+  std::mutex recorders_mu;
+  std::vector<cudaStream_t> recorders;
   // fault word of the kernels with bounded waits (pinned, mapped): nonzero once a
   // wait gave up; read and cleared by stream_sync
   unsigned* fault = nullptr;
 };
+
+// A stream to capture on, taken by one thread at a time and given back (creating and
+// destroying one costs 0.1 ms, as much as a captured pass of 128^3 adds to its first).
+int take_recorder(Context* c, cudaStream_t* stream);
+void give_recorder(Context* c, cudaStream_t stream);
 
 // Event pair around one launch of `kind` (no-op unless profiling); prof_end after the launch.
 int prof_begin(Context* c, int kind, cudaEvent_t* start);

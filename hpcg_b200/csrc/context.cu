@@ -275,6 +275,32 @@ int stream_sync(Context* c) {
   return HPCG_B200_OK;
 }
 
+int take_recorder(Context* c, cudaStream_t* stream) {
+  {
+    std::lock_guard<std::mutex> lock(c->recorders_mu);
+    if (!c->recorders.empty()) {
+      *stream = c->recorders.back();
+      c->recorders.pop_back();
+      return HPCG_B200_OK;
+    }
+  }
+  // not ordered with the legacy default stream: other threads may use that meanwhile
+  HB_CK(cudaStreamCreateWithFlags(stream, cudaStreamNonBlocking));
+  return HPCG_B200_OK;
+}
+
+void give_recorder(Context* c, cudaStream_t stream) {
+  constexpr size_t kKept = 4;
+  {
+    std::lock_guard<std::mutex> lock(c->recorders_mu);
+    if (c->recorders.size() < kKept) {
+      c->recorders.push_back(stream);
+      return;
+    }
+  }
+  cudaStreamDestroy(stream);
+}
+
 namespace {
 int take_event(Context* c, cudaEvent_t* e) {
   if (!c->ev_pool.empty()) {

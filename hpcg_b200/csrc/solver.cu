@@ -1101,7 +1101,10 @@ int run_captured(hpcg_b200_problem* p, cudaGraphExec_t& ex, F&& direct) {
     rec.scal = c->scal;
     rec.scal_host = c->scal_host;
     rec.fault = c->fault;
-    HB_CK(cudaStreamCreateWithFlags(&rec.stream, cudaStreamNonBlocking));
+    if (take_recorder(c, &rec.stream) != HPCG_B200_OK) {
+      cudaGetLastError();
+      return direct();
+    }
     cudaGraph_t g = nullptr;
     int st = HPCG_B200_OK;
     cudaError_t e = cudaStreamBeginCapture(rec.stream, cudaStreamCaptureModeThreadLocal);
@@ -1113,7 +1116,7 @@ int run_captured(hpcg_b200_problem* p, cudaGraphExec_t& ex, F&& direct) {
     }
     if (st == HPCG_B200_OK && e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
     if (g) cudaGraphDestroy(g);
-    cudaStreamDestroy(rec.stream);
+    give_recorder(c, rec.stream);
     if (st != HPCG_B200_OK || e != cudaSuccess) {  // refused: stream launches from now on
       cudaGetLastError();
       ex = nullptr;
