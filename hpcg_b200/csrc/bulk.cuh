@@ -331,7 +331,8 @@ __device__ __forceinline__ uint64_t evict_first_policy() {
 }
 // Before a block's first use of a tensor map that lies in global memory (not in the
 // kernel's parameters): the map is read through a proxy of its own, which may still
-// hold what an earlier map at the same address said.
+// hold what an earlier map at the same address said. (A batch of 16 problems: 0.1 of
+// 54 ms.)
 __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* m) {
   asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(m) : "memory");
 }
@@ -346,7 +347,7 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* m) {
 // the wait only the kernel directly before can have put lines there, and stale
 // ones are lines that it read and that another SM wrote meanwhile. `fence` drops
 // those too (0.2 us); a kernel may leave it out where no 32 bytes are read and
-// written by two blocks of the kernel before it.
+// written by two blocks of the kernel before it (GeoPhase::shared).
 __device__ __forceinline__ void griddep_wait(bool fence = true) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -298,10 +298,11 @@ int hpcg_b200_level_info(const hpcg_b200_problem* p, int level, int* nrow, int64
 
 /* Bytes of one level's packed column index, 0 if the level keeps only its
  * 32-bit columns (a 128-row tile whose columns of one slot span more than 65534,
- * or HPCG_B200_PACKED=0 at creation). One 7024-byte record per 128-row tile of
- * the storage: 27 32-bit bases, a word of padding and 27 x 128 16-bit offsets
- * (0xFFFF: the zero sink); the bulk-copy kernels read it instead of the 32-bit
- * columns, with the same column for every entry. */
+ * or HPCG_B200_PACKED=0 at creation). One record per 128-row tile of the storage:
+ * 27 32-bit bases, a word that names the form, and 27 x 128 sink bits (the diagonal
+ * form, 544 bytes), 8-bit offsets (3568) or 16-bit ones (7024). The bulk-copy kernels
+ * read it instead of the 32-bit columns, with the same column for every entry; on a
+ * level whose columns follow from its grid they read neither. */
 int hpcg_b200_level_packed(const hpcg_b200_problem* p, int level, int64_t* bytes);
 
 /* Copies one level's device layout to host: new2old[nrow] (colour row -> natural
